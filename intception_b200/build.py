@@ -1,6 +1,6 @@
 """Build libintception_b200.so in-tree for sm_100a.
 
-Steps: regenerate the device Boys table (mpmath), emit the per-class kernels,
+Steps: regenerate the device Boys and Rys tables (mpmath), emit the per-class kernels,
 compile every translation unit with nvcc in parallel, link one shared library.
 Outputs: intception_b200/libintception_b200.so; objects in intception_b200/_build/.
 
@@ -28,8 +28,9 @@ FLAGS = ['-O3', '-lineinfo', '-std=c++17', '-Xcompiler', '-fPIC', '--expt-relaxe
 def _generate():
     sys.path.insert(0, ROOT)
     import json
-    from intception_b200.emit import boys_table, eri_emitter
+    from intception_b200.emit import boys_table, eri_emitter, rys_table
     boys_table.write_headers(GEN)
+    rys_table.write_headers(GEN)
     stats = eri_emitter.emit_all(GEN)
     with open(os.path.join(PKG, 'class_stats.json'), 'w') as fh:
         json.dump(stats, fh, indent=0)

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "_gen/boys_table.h"
+#include "_gen/rys_table.h"
 
 #ifndef IB_BLOCK
 #define IB_BLOCK 128
@@ -44,6 +45,8 @@ struct IbLaunch {
   const double* prim_exp;
   const double* prim_coef;
   const double* boys_tab;  // [IB_BOYS_NPTS * IB_BOYS_NCOL]
+  const double* rys_tab;   // [IB_RYS_SIZE]
+  const double* boys_row;  // [IB_BOYS_ROW_LMAX + 1][IB_BOYS_NPTS][8] (ib_boys_row)
   const double* sph;       // library Cartesian->spherical matrices, packed per l
   double* out;
   int* status;             // device error word (0 = ok)
@@ -280,7 +283,7 @@ __device__ __forceinline__ unsigned ib_pin(unsigned x) {
   return y;
 }
 
-// Barrier over the n threads (64 or 128) of multi-warp lane group g of the
+// Barrier over the n threads (a multiple of 32) of multi-warp lane group g of the
 // block (named barrier g+1).
 __device__ __forceinline__ void ib_group_bar(int g, int n) {
   asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(n) : "memory");
@@ -770,6 +773,172 @@ __device__ __forceinline__ int2 ib_live_pairs_screened(const double* __restrict_
     n[side] = cnt;
   }
   return make_int2(n[0], n[1]);
+}
+
+// ---- Pieces of the warp-per-quartet kernels (emit/warp_emitter.py).
+
+// Pair data of primitive pair p = i0 * k1 + i1 of one side of the quartet:
+// zeta, 1/zeta, f = x1/zeta (the product centre lies at f along the line from
+// the first to the second shell) and c0 c1 exp(-x0 x1 R^2 / zeta) / zeta.
+// Returns whether the Gaussian factor is not zero.
+__device__ __forceinline__ bool ib_pair_values(const IbLaunch& a, const IbQuartet& g, int side, int p, double2& u,
+                                               double2& v) {
+  const int ptr0 = g.ptr[2 * side], ptr1 = g.ptr[2 * side + 1], k1 = g.k[2 * side + 1];
+  const double r2 = side ? g.RCD2 : g.RAB2;
+  const int i0 = p / k1, i1 = p - i0 * k1;
+  const double x0 = __ldg(a.prim_exp + ptr0 + i0), c0 = __ldg(a.prim_coef + ptr0 + i0);
+  const double x1 = __ldg(a.prim_exp + ptr1 + i1), c1 = __ldg(a.prim_coef + ptr1 + i1);
+  const double z = x0 + x1, oz = 1.0 / z;
+  const double K = ib_pair_factor(x0, c0, x1, c1, oz, r2);
+  u = make_double2(z, oz);
+  v = make_double2(x1 * oz, K * oz);
+  return K != 0.0;
+}
+__device__ __forceinline__ void ib_pair_data(const IbLaunch& a, const IbQuartet& g, int side, int p,
+                                             double* __restrict__ dst) {
+  double2 u, v;
+  ib_pair_values(a, g, side, p, u, v);
+  reinterpret_cast<double2*>(dst)[0] = u;
+  reinterpret_cast<double2*>(dst)[1] = v;
+}
+
+// Pair data of the live pairs (Gaussian factor not zero) among the n <= 64
+// pairs from p0, packed in increasing order; one warp; returns their number.
+__device__ __forceinline__ int ib_live_pair_data(const IbLaunch& a, const IbQuartet& g, int side, int p0, int n,
+                                                 double* __restrict__ dst, int lane) {
+  int cnt = 0;
+  for (int t0 = 0; t0 < n; t0 += 32) {
+    double2 u, v;
+    const bool live = t0 + lane < n && ib_pair_values(a, g, side, p0 + t0 + lane, u, v);
+    const unsigned bal = __ballot_sync(0xffffffffu, live);
+    if (live) {
+      double2* d = reinterpret_cast<double2*>(dst) + 2 * (cnt + __popc(bal & ((1u << lane) - 1u)));
+      d[0] = u;
+      d[1] = v;
+    }
+    cnt += __popc(bal);
+  }
+  return cnt;
+}
+
+// Geometry of one primitive quartet from its pair data.
+struct IbGeom {
+  double fb, fd, PQ[3], roz, roe, oz, oe, ozpe, T, pref;  // roz = rho/zeta, roe = rho/eta, oz = 1/zeta, ...
+};
+__device__ __forceinline__ void ib_geometry(const double* __restrict__ pab, const double* __restrict__ pcd,
+                                            const IbQuartet& g, IbGeom& o) {
+  const double2 ab0 = reinterpret_cast<const double2*>(pab)[0], ab1 = reinterpret_cast<const double2*>(pab)[1];
+  const double2 cd0 = reinterpret_cast<const double2*>(pcd)[0], cd1 = reinterpret_cast<const double2*>(pcd)[1];
+  const double zeta = ab0.x, eta = cd0.x;
+  const double rs = rsqrt(zeta + eta);
+  o.ozpe = rs * rs;
+  o.roz = eta * o.ozpe;
+  o.roe = zeta * o.ozpe;
+  double r2 = 0.0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double P = fma(-ab1.x, g.AB[d], g.A[d]), Q = fma(-cd1.x, g.CD[d], g.C[d]);
+    o.PQ[d] = P - Q;
+    r2 = fma(o.PQ[d], o.PQ[d], r2);
+  }
+  o.fb = ab1.x;
+  o.fd = cd1.x;
+  o.oz = ab0.y;
+  o.oe = cd0.y;
+  o.T = zeta * o.roz * r2;
+  o.pref = ib_two_pi52() * rs * ab1.y * cd1.y;
+}
+
+// The same for the Rys steps, into shared memory, 32 doubles apart: fb, P - Q
+// (3), rho/zeta, rho/eta, 1/2zeta, 1/2eta, 1/2(zeta+eta), T, the prefactor, fd.
+__device__ __forceinline__ void ib_rys_setup(const double* __restrict__ pab, const double* __restrict__ pcd,
+                                             const IbQuartet& g, double* __restrict__ o) {
+  IbGeom q;
+  ib_geometry(pab, pcd, g, q);
+  o[0 * 32] = q.fb;
+  o[1 * 32] = q.PQ[0];
+  o[2 * 32] = q.PQ[1];
+  o[3 * 32] = q.PQ[2];
+  o[4 * 32] = q.roz;
+  o[5 * 32] = q.roe;
+  o[6 * 32] = 0.5 * q.oz;
+  o[7 * 32] = 0.5 * q.oe;
+  o[8 * 32] = 0.5 * q.ozpe;
+  o[9 * 32] = q.T;
+  o[10 * 32] = q.pref;
+  o[11 * 32] = q.fd;
+}
+
+// F_0..F_L(T) for the lane-per-primitive kernels.  Row i of L holds F_(L+k)(T_i)/k!,
+// k = 0..6, and exp(-T_i), T_i = i/16: 64 bytes, four 16-byte loads.  A warp's
+// lanes hit 32 unrelated rows, and the gather is what bounds this function:
+// 79 SM cycles a warp this way, 220-250 with seven 8-byte loads from 256-byte
+// rows.  exp(-T) = exp(-T_i) times the Taylor sum of exp(T_i - T) (|.| <= 1/32,
+// degree 7: 3e-17).  Above the table: F_0 = sqrt(pi/T)/2 and upward recursion;
+// its exp(-T) matters to F_5(36) by 3e-11 relative and less beyond, so float
+// is enough up to L = 5.
+#define IB_BOYS_ROW_LMAX 8
+template <int L>
+__device__ __forceinline__ void ib_boys_row(double T, const double* __restrict__ tab, double* F) {
+  if (T < IB_BOYS_TMAX) {
+    const int i = __double2int_rn(T * (double)IB_BOYS_H_INV);
+    const double dx = fma((double)i, 1.0 / IB_BOYS_H_INV, -T);
+    const double2* __restrict__ r = reinterpret_cast<const double2*>(tab) + ((size_t)L * IB_BOYS_NPTS + i) * 4;
+    const double2 c0 = __ldg(r), c1 = __ldg(r + 1), c2 = __ldg(r + 2), c3 = __ldg(r + 3);
+    double f = fma(c3.x, dx, c2.y);
+    f = fma(f, dx, c2.x);
+    f = fma(f, dx, c1.y);
+    f = fma(f, dx, c1.x);
+    f = fma(f, dx, c0.y);
+    F[L] = fma(f, dx, c0.x);
+    if (L > 0) {
+      double e = fma(dx, 1.0 / 5040.0, 1.0 / 720.0);
+      e = fma(e, dx, 1.0 / 120.0);
+      e = fma(e, dx, 1.0 / 24.0);
+      e = fma(e, dx, 1.0 / 6.0);
+      e = fma(e, dx, 0.5);
+      e = fma(e, dx, 1.0);
+      e = fma(e, dx, 1.0) * c3.y;
+      const double t2 = T + T;
+#pragma unroll
+      for (int m = L - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], e) * (1.0 / (2 * m + 1));
+    }
+  } else {
+    const double r = rsqrt(T), oT = r * r;
+    F[0] = 0.88622692545275801365 * r;  // sqrt(pi)/2 T^-1/2
+    if (L > 0) {
+      const double he = L <= 5 ? 0.5 * (double)expf(-(float)T) : 0.5 * exp(-T);
+#pragma unroll
+      for (int m = 0; m < L; ++m) F[m + 1] = fma((double)m + 0.5, F[m], -he) * oT;
+    }
+  }
+}
+
+// Root rt of N at Boys argument T: (u, weight x pref).
+template <int N>
+__device__ __forceinline__ void ib_rys_root(const double* __restrict__ tab, double T, double pref, int rt,
+                                            double* __restrict__ dst) {
+  const double2* __restrict__ t = reinterpret_cast<const double2*>(tab + ib_rys_off(N)) + rt;
+  double2 v;
+  if (T < (double)ib_rys_tmax(N)) {
+    const double s = T * (double)IB_RYS_H_INV;
+    const int row = (int)s;
+    const double x = fma(2.0, s - (double)row, -1.0);
+    t += row * ((IB_RYS_DEG + 1) * N);
+    v = __ldg(t + IB_RYS_DEG * N);
+#pragma unroll
+    for (int k = IB_RYS_DEG - 1; k >= 0; --k) {
+      const double2 c = __ldg(t + k * N);
+      v.x = fma(v.x, x, c.x);
+      v.y = fma(v.y, x, c.y);
+    }
+  } else {
+    const double2 c = __ldg(t + ib_rys_tmax(N) * IB_RYS_H_INV * (IB_RYS_DEG + 1) * N);
+    const double r = rsqrt(T);
+    v.x = c.x * r * r;
+    v.y = c.y * r;
+  }
+  reinterpret_cast<double2*>(dst)[0] = make_double2(v.x, v.y * pref);
 }
 
 template <typename R>

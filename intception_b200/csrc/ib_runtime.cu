@@ -26,6 +26,7 @@
 
 #include "../../include/intception_b200.h"
 #include "_gen/boys_table_data.h"
+#include "_gen/rys_table_data.h"
 #include "ib_eri_device.cuh"
 #include "ib_generic.cuh"
 
@@ -132,7 +133,7 @@ struct Context {
   double hrr_tol = 1e-13;
   cudaStream_t side[kNSideMax] = {};
   cudaEvent_t fork = nullptr, join[kNSideMax] = {};
-  DevBuf boys_tab, sph, keys, vals, keys2, vals2, items, ranges, status, cub_tmp, scratch;
+  DevBuf boys_tab, rys_tab, boys_row, sph, keys, vals, keys2, vals2, items, ranges, status, cub_tmp, scratch;
   DevBuf counters;  // per class kernel launch of a batch: the next quartet (FP64, FP32, FP64 recheck passes)
   DevBuf sw_quartets, sw_sizes, sw_off, sw_tmp, sw_blocks;  // Schwarz-bound work buffers
   DevBuf flags;    // per sorted item of the last batch: FP32 rejection (bit 0), on the redo list (bit 1)
@@ -537,6 +538,21 @@ int get_context(Context** out) {
     IB_CUDA(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
     IB_CUDA(c->boys_tab.ensure(sizeof(ib_boys_host_table)));
     IB_CUDA(cudaMemcpy(c->boys_tab.p, ib_boys_host_table, sizeof(ib_boys_host_table), cudaMemcpyHostToDevice));
+    IB_CUDA(c->rys_tab.ensure(sizeof(ib_rys_host_table)));
+    IB_CUDA(cudaMemcpy(c->rys_tab.p, ib_rys_host_table, sizeof(ib_rys_host_table), cudaMemcpyHostToDevice));
+    std::vector<double> rows((size_t)(IB_BOYS_ROW_LMAX + 1) * IB_BOYS_NPTS * 8);
+    for (int L = 0; L <= IB_BOYS_ROW_LMAX; ++L)
+      for (int i = 0; i < IB_BOYS_NPTS; ++i) {
+        double* row = rows.data() + ((size_t)L * IB_BOYS_NPTS + i) * 8;
+        double fact = 1.0;
+        for (int k = 0; k < IB_BOYS_TAYLOR; ++k) {
+          row[k] = ib_boys_host_table[i * IB_BOYS_NCOL + L + k] / fact;
+          fact *= k + 1;
+        }
+        row[7] = std::exp(-(double)i / IB_BOYS_H_INV);
+      }
+    IB_CUDA(c->boys_row.ensure(rows.size() * sizeof(double)));
+    IB_CUDA(cudaMemcpy(c->boys_row.p, rows.data(), rows.size() * sizeof(double), cudaMemcpyHostToDevice));
     std::vector<double> sph;
     build_sph_host(sph);
     IB_CUDA(c->sph.ensure(sph.size() * sizeof(double)));
@@ -571,6 +587,8 @@ IbLaunch base_launch(Context* c) {
   IbLaunch a;
   std::memset(&a, 0, sizeof(a));
   a.boys_tab = c->boys_tab.as<double>();
+  a.rys_tab = c->rys_tab.as<double>();
+  a.boys_row = c->boys_row.as<double>();
   a.sph = c->sph.as<double>();
   a.status = c->status.as<int>();
   a.slice_boost = c->slice_boost;

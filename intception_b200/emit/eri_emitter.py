@@ -37,7 +37,6 @@ from intception_b200.basis import sph_matrix  # noqa: E402
 LMAX_EMIT = 2  # classes with every l <= LMAX_EMIT get an unrolled kernel
 # classes kept on the one-thread-per-quartet kernel (everything else whose
 # smaller side fits a warp uses the lane-group kernel of group_emitter.py)
-THREAD_CLASSES = set()
 
 DIRS = 'xyz'
 NPAIR_TOTAL = 7 * 8 // 2                       # shell pairs with l <= 6 (IB_NPAIR)
@@ -388,27 +387,6 @@ class Emitter:
         src.append('  }')
         src.append('}')
         src.append('')
-        # host-side launcher and occupancy query for this class
-        src.append('static void ib_launch_%s(int variant, int grid, cudaStream_t s, const IbLaunch& a) {' % t)
-        src.append('  const size_t smem = 0;')
-        src.append('  switch (variant) {')
-        src.append('    case 0: ib_eri_%s<double, false><<<grid, IB_BLOCK, smem, s>>>(a); break;' % t)
-        src.append('    case 1: ib_eri_%s<double, true><<<grid, IB_BLOCK, smem, s>>>(a); break;' % t)
-        src.append('    case 2: ib_eri_%s<float, false><<<grid, IB_BLOCK, smem, s>>>(a); break;' % t)
-        src.append('    default: ib_eri_%s<float, true><<<grid, IB_BLOCK, smem, s>>>(a); break;' % t)
-        src.append('  }')
-        src.append('}')
-        src.append('static int ib_occupancy_%s(int variant) {' % t)
-        src.append('  int n = 0; const size_t smem = 0;')
-        src.append('  switch (variant) {')
-        src.append('    case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ib_eri_%s<double, false>, IB_BLOCK, smem); break;' % t)
-        src.append('    case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ib_eri_%s<double, true>, IB_BLOCK, smem); break;' % t)
-        src.append('    case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ib_eri_%s<float, false>, IB_BLOCK, smem); break;' % t)
-        src.append('    default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ib_eri_%s<float, true>, IB_BLOCK, smem); break;' % t)
-        src.append('  }')
-        src.append('  return n;')
-        src.append('}')
-        src.append('')
         stats = dict(tag=t, cid=cid, L=L, nodes=self.nvar, vrr_flops=self.flops, hrr_flops=self.hrr_flops,
                      sph_flops=sph_flops, nacc=nacc)
         return '\n'.join(src), stats
@@ -421,56 +399,84 @@ DEFAULT_SLICE_CAP = 8
 SMEM_LIMIT = 227 * 1024
 
 
-def group_fits(c):
-    """Whether class c gets a lane-group kernel: the smaller side fits a
-    128-lane group, its base-chain path has at most 6 steps (the lane code
-    packs 6), and a block's shared memory stays within SMEM_LIMIT."""
-    from .group_emitter import GroupEmitter, orientation
-    if orientation(*c) is None or min(c[0] + c[1], c[2] + c[3]) > 6:
-        return False
-    g = GroupEmitter(*c)
-    g.kernel(fp32=False)
-    groups = (128 // g.G) if g.wide else 4 * g.QPW
-    return groups * g.per_group * 8 <= SMEM_LIMIT
+def thread_class(c):
+    """Whether class c's FP64 kernel evaluates a primitive quartet per lane
+    (warp_emitter.ThreadEmitter): every ket without angular momentum, and the
+    other classes whose [e0|f0] table fits a lane's registers beside the
+    recurrence."""
+    n = 1
+    for l0, l1 in ((c[0], c[1]), (c[2], c[3])):
+        n *= len(comps_range(l0, l0 + l1))
+    return c[2] + c[3] == 0 or n <= THREAD_TARGETS
+
+
+THREAD_TARGETS = 60
+
+
+def fp64_emitter(c):
+    from .warp_emitter import RysEmitter, ThreadEmitter
+    return ThreadEmitter(*c) if thread_class(c) else RysEmitter(*c)
+
+
+def class_fits(c):
+    """Whether class c gets an unrolled kernel: a block's shared memory stays
+    within SMEM_LIMIT, and a lane-per-primitive kernel has at most 100
+    accumulators ((gg|ss) has 145)."""
+    e = fp64_emitter(c)
+    e.kernel()
+    return e.smem <= SMEM_LIMIT and e.nacc() <= 100
 
 
 def emitted_classes():
-    """Canonical classes with an unrolled kernel: every class with l <= 2
-    (FP64 and FP32-VRR variants), and every class with an f or g shell and the
-    rest <= g that group_fits (FP64 only; the nuclear-gradient batches of an
-    l <= 2 basis reach the one-f classes, an f basis the rest of the f
-    classes, l <= 4 bases the g classes).  (gf|gf), (gg|gf), (gg|gg) and
-    (gg|ss) stay on the generic kernel."""
+    """Canonical classes with an unrolled kernel, and whether they have FP32
+    variants: every class with l <= 2 (FP64 and FP32-VRR), and every class with
+    an f or g shell and the rest <= g whose kernel fits (FP64 only; the
+    nuclear-gradient batches of an l <= 2 basis reach the one-f classes, an f
+    basis the rest of the f classes, l <= 4 bases the g classes)."""
     out = [(c, True) for c in canonical_classes(LMAX_EMIT)]
     for c in canonical_classes(4):
-        if max(c) >= 3 and group_fits(c):
+        if max(c) >= 3 and class_fits(c):
             out.append((c, False))
     # the reversed (d f| pair against every pair up to f (bra: its pair id is the largest)
     for kp in [(a, b) for a in range(4) for b in range(a + 1)] + [(2, 3)]:
         c = (2, 3) + kp
-        if group_fits(c):
+        if class_fits(c):
             out.append((c, False))
     out.sort(key=lambda x: class_id(*x[0]))
     return out
 
 
-def emit_all(outdir, lmax=LMAX_EMIT, ngroups=8):
+def class_source(c, fp32):
+    """CUDA source of class c (its kernels, launcher and occupancy query) and
+    its statistics."""
+    from .group_emitter import GroupEmitter, launcher
+    e = fp64_emitter(c)
+    parts = [e.kernel()]
+    only = None if max(c) <= 2 else e.budget()
+    kernels = [('%s<%s, %%d>' % (e.name, S), e.block, e.smem, only) for S in ('false', 'true')]
+    if fp32:
+        g = GroupEmitter(*c)
+        parts.append(g.kernel()[0])
+        kernels += [('ib_eri_%s<float, %s, %%d>' % (g.tag, S), 'IB_BLOCK', g.smem_bytes, None)
+                    for S in ('false', 'true')]
+    else:
+        kernels *= 2
+    parts.append(launcher(e.tag, kernels))
+    return '\n'.join(parts), dict(kind=e.kind, G=e.G, budget=e.budget())
+
+
+def emit_all(outdir, lmax=LMAX_EMIT, ngroups=24):
     """Write the class translation units and the dispatch table into outdir.
     Returns the list of per-class statistics."""
     os.makedirs(outdir, exist_ok=True)
     classes = emitted_classes()
     # balance translation units by emitted size (largest classes first)
-    from .group_emitter import GroupEmitter, orientation
     bodies = []
     for c, fp32 in classes:
         # the one-thread schedule's counts are the algorithmic work of the class
-        tbody, st = Emitter(*c).kernel()
-        if orientation(*c) is not None and c not in THREAD_CLASSES:
-            body, gst = GroupEmitter(*c).kernel(fp32=fp32)
-            st.update(kind='group', G=gst['G'], orient=gst['orient'], lane_flops=gst['lane_flops'])
-        else:
-            body = tbody
-            st['kind'] = 'thread'
+        st = Emitter(*c).kernel()[1]
+        body, gst = class_source(c, fp32)
+        st.update(gst)
         st['fp32'] = fp32
         bodies.append((c, body, st))
     order = sorted(bodies, key=lambda x: -len(x[1]))
@@ -508,7 +514,8 @@ def emit_all(outdir, lmax=LMAX_EMIT, ngroups=8):
     # python -m intception_b200.autotune on a GPU): per class and variant the
     # register-budget index, per class the slice cap and whether the FP32 tier
     # uses the class's FP32 kernel (where it measured faster than FP64)
-    minb = [[0] * 4 for _ in range(NCLASS_TOTAL)]
+    budget = {b[2]['cid']: b[2]['budget'] for b in bodies}
+    minb = [[budget.get(cid) or 0] * 2 + [0] * 2 for cid in range(NCLASS_TOTAL)]
     # at most 8 lane groups per quartet unless tuned otherwise: measured on the
     # screened l <= 2 step (3.4 % of 1e6 quartets kept, primitive screening at
     # 1e-18), a cap of 8 gave 1.18 ms per step against 1.30 uncapped, 1.36 at 2
@@ -523,6 +530,7 @@ def emit_all(outdir, lmax=LMAX_EMIT, ngroups=8):
         for tag, ent in tun.get('classes', {}).items():
             cid = class_id(*(int(ch) for ch in tag))
             minb[cid] = [int(x) for x in ent.get('minb', [0, 0, 0, 0])]
+            minb[cid][:2] = ent.get('warp_minb', [budget[cid]] * 2)
             scap[cid] = int(ent.get('slice_cap', DEFAULT_SLICE_CAP))
             fp32on[cid] = 1 if ent.get('fp32', True) else 0
     disp.append('extern const int ib_tuned_minb[%d][4] = {%s};'

@@ -451,6 +451,9 @@ class GroupEmitter:
         nc = (2 * lc + 1) if sph else len(Cc)
         nd = (2 * ld + 1) if sph else len(D)
         L = []
+        if self.split_bra():
+            base, size = self.emit_bra_split(sph, NF, NFP, L)
+            return L + self.emit_ket(sph, na, nb, nc, nd, Flist, NF, NFP, base), size
         # bra HRR, lanes over f
         L.append('    for (int t = r; t < %d; t += SG) {' % NF)
         for e in range(NE):
@@ -471,11 +474,23 @@ class GroupEmitter:
             L.append('      sb0[%d * %d + t] = %s;' % (u, NFP, name))
         L.append('    }')
         L.append('    ib_sg_sync(SG, sg, sgmask);')
-        # ket HRR, lanes over ab
+        L += self.emit_ket(sph, na, nb, nc, nd, Flist, NF, NFP, 0)
+        return L, max(NE, len(A) * len(B)) * NFP
+
+    def split_bra(self):
+        """Whether the bra HRR runs over (f, a) lanes (emit_bra_split)."""
+        return False
+
+    def emit_ket(self, sph, na, nb, nc, nd, Flist, NF, NFP, base):
+        """Ket HRR, transform and store; the table [ab][f] starts at base."""
+        lc, ld = self.lc, self.ld
+        Cc, D = comps(lc), comps(ld)
+        f_index = {f: i for i, f in enumerate(Flist)}
+        L = []
         NAB = na * nb
         L.append('    for (int u = r; u < %d; u += SG) {' % NAB)
         for f in range(NF):
-            L.append('      const double w%d = sb0[u * %d + %d];' % (f, NFP, f))
+            L.append('      const double w%d = sb0[%d + u * %d + %d];' % (f, base, NFP, f))
         body = []
         cnt = [0]
         res = self._hrr(Cc, D, lambda c: 'w%d' % f_index[c], 'CD', 'k', body, cnt)
@@ -494,7 +509,7 @@ class GroupEmitter:
             off = ' + '.join(x for x in (('%d * g.st[2]' % i) if i else '', ('%d * g.st[3]' % k) if k else '') if x)
             L.append('      ou[%s] = %s;' % (off or '0', name))
         L.append('    }')
-        return L, max(NE, len(A) * len(B)) * NFP
+        return L
 
     def err_expr(self):
         """FP32 error bound of the primitive quartet held in pq/F (see ib_fp32_err)."""
@@ -555,8 +570,8 @@ class GroupEmitter:
         bb, wb = weights(self.la, self.lb, 'rab')
         bd, wd = weights(self.lc, self.ld, 'rcd')
         out = ['    if (a.hrr_tol > 0.0) {',
-               '      const double rab = sqrt(g.AB[0] * g.AB[0] + g.AB[1] * g.AB[1] + g.AB[2] * g.AB[2]);',
-               '      const double rcd = sqrt(g.CD[0] * g.CD[0] + g.CD[1] * g.CD[1] + g.CD[2] * g.CD[2]);',
+               '      // distances in float (an estimate; rounded up by 1e-6)',
+               '      const double rab = 1.000001 * (double)sqrtf((float)g.RAB2), rcd = 1.000001 * (double)sqrtf((float)g.RCD2);',
                '      (void)rab; (void)rcd;',
                '      double hm = 0.0;',
                '      for (int x = r; x < %d; x += SG) {' % (NE * NF),
@@ -565,13 +580,14 @@ class GroupEmitter:
                                                                           select('col', bd, wd)),
                '      }',
                '      if (hm * IB_HRR_ERR_COEF > a.hrr_tol) ib_redo_push(a, p);',
+               '      ib_sg_sync(SG, sg, sgmask);  // the whole table is read before the HRR overwrites it',
                '    }']
         return out
 
     # -------------------------------------------------------------- kernel
-    def kernel(self, fp32=True):
-        """CUDA source of the class kernel and its launcher; fp32=False
-        instantiates the FP64 variants only (FP32 requests run in FP64)."""
+    def kernel(self):
+        """CUDA source of the class kernel (template over the VRR's type, the
+        output kind and the register budget)."""
         chain, NT = self.emit_chain()
         epi_cart, sm_cart = self.emit_epilogue(False)
         epi_sph, sm_sph = self.emit_epilogue(True)
@@ -984,40 +1000,33 @@ class GroupEmitter:
             smem_bytes = '(sizeof(double) * (IB_BLOCK / %d) * %d)' % (self.G, per_group)
         else:
             smem_bytes = '(sizeof(double) * (IB_BLOCK / 32) * %d * %d)' % (self.QPW, per_group)
-        src.append('static size_t ib_smem_%s() { return %s; }' % (t, smem_bytes))
-        # variant = v4 + 4 * mi: v4 = precision x output (FP64/FP32 x Cartesian/
-        # spherical), mi indexes the register budget IB_MINB[mi] (minimum
-        # resident blocks per SM); classes outside the tuned set instantiate
-        # mi = 0 only
-        variants = (('double', 'false'), ('double', 'true'), ('float', 'false'), ('float', 'true'))
-        if not fp32:
-            variants = variants[:2] * 2
-        minbs = list(range(len(MINB_VALUES))) if self.tuned else [0]
-        cases = []
-        for mi in range(len(MINB_VALUES)):
-            for v, (R, S) in enumerate(variants):
-                use = mi if mi in minbs else 0
-                cases.append((v + 4 * mi, 'ib_eri_%s<%s, %s, %d>' % (t, R, S, MINB_VALUES[use])))
-        src.append('static void ib_launch_%s(int variant, int grid, cudaStream_t s, const IbLaunch& a) {' % t)
-        src.append('  const size_t smem = ib_smem_%s();' % t)
-        src.append('  switch (variant) {')
-        for v, fn in cases:
-            src.append('    case %d: %s<<<grid, IB_BLOCK, smem, s>>>(a); break;' % (v, fn))
-        src.append('  }')
-        src.append('}')
-        src.append('static int ib_occupancy_%s(int variant) {' % t)
-        src.append('  int n = 0; const size_t smem = ib_smem_%s();' % t)
-        src.append('  switch (variant) {')
-        for v, fn in cases:
-            src.append('    case %d: cudaFuncSetAttribute(%s, cudaFuncAttributeMaxDynamicSharedMemorySize, '
-                       '(int)smem); cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, %s, IB_BLOCK, '
-                       'smem); break;' % (v, fn, fn))
-        src.append('  }')
-        src.append('  return n;')
-        src.append('}')
-        src.append('')
+        self.smem_bytes = smem_bytes
         # the group barrier counts the group's G threads (named barrier gid + 1)
         src = [ln.replace('ib_group_bar(gid)', 'ib_group_bar(gid, %d)' % self.G) for ln in src]
         stats = dict(tag=t, cid=self.cid, L=L, kind='group', G=self.G, orient=self.orient, nodes=self.nvar,
                      lane_flops=self.flops, nacc=NE * NF)
         return '\n'.join(src), stats
+
+
+def launcher(tag, kernels):
+    """Host launcher and occupancy query of a class.  kernels: for the four
+    variants v4 (FP64/FP32 x Cartesian/spherical) the kernel's name with its
+    template arguments up to the register budget, its threads per block, its
+    shared-memory size, and the one budget that is instantiated (None: all).
+    variant = v4 + 4 * mi, mi the register budget MINB_VALUES[mi] (minimum
+    resident blocks per SM)."""
+    cases = []
+    for mi in range(len(MINB_VALUES)):
+        for v, (fn, block, smem, only) in enumerate(kernels):
+            cases.append((v + 4 * mi, fn % MINB_VALUES[mi if only is None else only], block, smem))
+    src = ['static void ib_launch_%s(int variant, int grid, cudaStream_t s, const IbLaunch& a) {' % tag,
+           '  switch (variant) {']
+    for v, fn, block, smem in cases:
+        src.append('    case %d: %s<<<grid, %s, %s, s>>>(a); break;' % (v, fn, block, smem))
+    src += ['  }', '}', 'static int ib_occupancy_%s(int variant) {' % tag, '  int n = 0;', '  switch (variant) {']
+    for v, fn, block, smem in cases:
+        src.append('    case %d: cudaFuncSetAttribute(%s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)%s); '
+                   'cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, %s, %s, %s); break;'
+                   % (v, fn, smem, fn, block, smem))
+    src += ['  }', '  return n;', '}', '']
+    return '\n'.join(src)
