@@ -27,6 +27,10 @@
 #define IB_NPAIR_EXT (IB_NPAIR + 1)
 #define IB_NCLASS (IB_NPAIR_EXT * (IB_NPAIR_EXT + 1) / 2)
 #define IB_BOYS_TAYLOR 7
+// ranges: FP64 and FP32 [begin, end) per class, three more pairs, then the end
+// of each class's FP64 quartets of at least 2^IB_MERGED_LONG_LOG2 primitive quartets
+#define IB_SLOT_LONG_END (4 * IB_NCLASS + 6)
+#define IB_MERGED_LONG_LOG2 7
 
 struct IbItem {
   int s[4];         // shells (a, b, c, d) in canonical order
@@ -125,6 +129,30 @@ int ib_generic_split();
 int ib_generic_bps();
 cudaError_t ib_generic_launch(int grid, cudaStream_t s, const IbLaunch& a, const IbGenWork& wk, int sph,
                               double* scratch, long long slice);
+
+__device__ __forceinline__ int ib_ncart_d(int l) { return (l + 1) * (l + 2) / 2; }
+__device__ __forceinline__ int ib_pair_d(int la, int lb) { return la * (la + 1) / 2 + lb; }
+
+// canonical order: (a,b) with la>=lb, (c,d) with lc>=ld, bra pair index >= ket pair index
+__device__ __forceinline__ void ib_canon(int* s, int* l, int* st) {
+  if (l[0] < l[1]) {
+    int t = s[0]; s[0] = s[1]; s[1] = t;
+    t = l[0]; l[0] = l[1]; l[1] = t;
+    t = st[0]; st[0] = st[1]; st[1] = t;
+  }
+  if (l[2] < l[3]) {
+    int t = s[2]; s[2] = s[3]; s[3] = t;
+    t = l[2]; l[2] = l[3]; l[3] = t;
+    t = st[2]; st[2] = st[3]; st[3] = t;
+  }
+  if (ib_pair_d(l[0], l[1]) < ib_pair_d(l[2], l[3])) {
+    for (int k = 0; k < 2; ++k) {
+      int t = s[k]; s[k] = s[k + 2]; s[k + 2] = t;
+      t = l[k]; l[k] = l[k + 2]; l[k + 2] = t;
+      t = st[k]; st[k] = st[k + 2]; st[k + 2] = t;
+    }
+  }
+}
 
 // Smallest primitive exponent of shell s.
 __device__ __forceinline__ double ib_min_exp(const int* __restrict__ shell_k, const int* __restrict__ shell_ptr,
@@ -503,8 +531,8 @@ struct IbQuartet {
   long long off;
 };
 
-__device__ __forceinline__ void ib_load_quartet(const IbLaunch& a, int p, IbQuartet& g) {
-  const IbItem it = a.items[p];
+__device__ __forceinline__ void ib_load_quartet(const IbLaunch& a, const IbItem& item, IbQuartet& g) {
+  const IbItem it = item;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int s = it.s[i];

@@ -10,6 +10,7 @@
 //                      the [begin,end) range of every (precision, class)
 //   4. per-class persistent kernels (unrolled, emitted) fanned out over side
 //      streams, plus the generic block-per-quartet kernel for the rest.
+// A small FP64 batch with every l <= 2 takes one kernel instead (ib_small.cuh).
 // The drop-ins build the same items on the host for one quartet (all
 // contraction combinations) and reuse the class kernels.
 #include <cuda_runtime.h>
@@ -29,6 +30,7 @@
 #include "_gen/rys_table_data.h"
 #include "ib_eri_device.cuh"
 #include "ib_generic.cuh"
+#include "ib_small.cuh"
 
 void ib_register_emitted_classes(IbClassEntry* table);
 // Real solid harmonics in the library convention (m = -l..l, each scaled to the
@@ -47,12 +49,22 @@ constexpr int kSlotFp32 = 2 * IB_NCLASS;        // ranges offset of the FP32 cop
 constexpr int kSlotGenHeavy = 4 * IB_NCLASS;    // [begin, end) of the generic kernel's heavy quartets
 constexpr int kSlotSkip = 4 * IB_NCLASS + 2;    // [begin, end) of the screened-out quartets
 constexpr int kSlotGenLight = 4 * IB_NCLASS + 4;  // [begin, end) of the generic kernel's light quartets
-constexpr int kNRanges = 4 * IB_NCLASS + 6;
+constexpr int kNRanges = IB_SLOT_LONG_END + IB_NCLASS;
 constexpr int kNCounters = 3 * IB_NCLASS;      // quartet counters: FP64 pass, FP32 pass, FP64 recheck pass
 // sort key: skip(1) generic(1) fp32(1) class(9) work(4), two radix passes; a
 // generic quartet's class and work bits hold light(1) and its cost code (8)
 constexpr int kKeyBits = 16;
 constexpr size_t kScratchCap = size_t(4) << 30;  // bytes of generic-kernel scratch at most
+// FP64 batches with every l <= 2.  Up to kSmallBatch quartets: the small-batch
+// kernel (us per batch, against the fan-out of one kernel per class: 256
+// quartets of K <= 3 41 / 107, of K <= 6 94 / 108; one block per quartet).  Up
+// to kMergedBatch, when the batch has d shells: the sorted pipeline with the
+// class kernels merged into one launch (1 200 quartets 64 / 106 and 97 / 107,
+// 2 400 103 / 110 and 124 / 132; level at 4 096, where the fan-out's register
+// budgets per class start to win).  Without d shells the fan-out is six
+// launches and as fast from 600 quartets on.
+constexpr int kSmallBatch = 296;
+constexpr int kMergedBatch = 3072;
 constexpr int kRedoGroups = 4;  // redo lists of an l >= 3 batch (dispatch)
 constexpr int kTickets = 2 * (1 + kRedoGroups);  // generic-kernel ticket pairs: the range launch, each redo list
 // blocks per cluster sharing a heavy generic quartet: a redo list is short and
@@ -136,8 +148,15 @@ struct Context {
   DevBuf boys_tab, rys_tab, boys_row, sph, keys, vals, keys2, vals2, items, ranges, status, cub_tmp, scratch;
   DevBuf counters;  // per class kernel launch of a batch: the next quartet (FP64, FP32, FP64 recheck passes)
   DevBuf sw_quartets, sw_sizes, sw_off, sw_tmp, sw_blocks;  // Schwarz-bound work buffers
+  std::vector<int> classes;  // emitted class ids, the heaviest first (descending id)
+  std::vector<int> lmax_of;  // their largest l
   DevBuf flags;    // per sorted item of the last batch: FP32 rejection (bit 0), on the redo list (bit 1)
   int flags_nq = 0;  // its quartet count (flags beyond it are stale)
+  // the small-batch kernel's control words and items, sized once for the largest such batch
+  DevBuf small_ctl, small_items;
+  const int* last_status = nullptr;  // status word and redo list of the last batch
+  const int* last_redo = nullptr;    // (null after a drop-in call: the host copies)
+  int host_status = 0, host_redo = 0;
   DevBuf redo;     // the last batch's redo lists (redo_groups of them, redo_stride ints apart; IbLaunch::redo)
   int redo_groups = 1, redo_stride = 2;
   DevBuf tickets;  // kTickets ints: the generic kernel's ticket pairs (zeroed by every dispatch)
@@ -156,30 +175,6 @@ std::mutex g_ctx_mu;
 
 // ---------------------------------------------------------------- kernels
 
-__device__ __forceinline__ int ib_ncart_d(int l) { return (l + 1) * (l + 2) / 2; }
-__device__ __forceinline__ int ib_pair_d(int la, int lb) { return la * (la + 1) / 2 + lb; }
-
-// canonical order: (a,b) with la>=lb, (c,d) with lc>=ld, bra pair index >= ket pair index
-__device__ __forceinline__ void ib_canon(int* s, int* l, int* st) {
-  if (l[0] < l[1]) {
-    int t = s[0]; s[0] = s[1]; s[1] = t;
-    t = l[0]; l[0] = l[1]; l[1] = t;
-    t = st[0]; st[0] = st[1]; st[1] = t;
-  }
-  if (l[2] < l[3]) {
-    int t = s[2]; s[2] = s[3]; s[3] = t;
-    t = l[2]; l[2] = l[3]; l[3] = t;
-    t = st[2]; st[2] = st[3]; st[3] = t;
-  }
-  if (ib_pair_d(l[0], l[1]) < ib_pair_d(l[2], l[3])) {
-    for (int k = 0; k < 2; ++k) {
-      int t = s[k]; s[k] = s[k + 2]; s[k + 2] = t;
-      t = l[k]; l[k] = l[k + 2]; l[k + 2] = t;
-      t = st[k]; st[k] = st[k + 2]; st[k + 2] = t;
-    }
-  }
-}
-
 // ib_reverse_for_classes out of line: classify runs it for every evaluated
 // quartet but it rarely does anything, and inlined its registers would lower
 // the occupancy of the whole (gather-latency-bound) kernel.
@@ -190,12 +185,24 @@ __device__ __noinline__ int ib_reverse_noinline(const int* __restrict__ shell_k,
   return ib_reverse_for_classes(shell_k, shell_ptr, prim_exp, shell_xyz, s, l, st, fd_only);
 }
 
+struct IbZeroed {  // zeroed by ib_classify: ranges, counters, tickets, the redo lists' counts, flags [nq]
+  int *ranges, *counters, *tickets, *redo, *flags;
+  int nranges, ncounters, ntickets, redo_groups, redo_stride;
+};
+
 __global__ void ib_classify(const int* __restrict__ quartets, const int* __restrict__ shell_l,
                             const int* __restrict__ shell_k, const int* __restrict__ shell_ptr,
                             const double* __restrict__ prim_exp, const double* __restrict__ shell_xyz, int nq,
                             int lmax, const double* __restrict__ bounds, double skip_below, double thr, int mixed,
                             const int* __restrict__ kind, int route_rev, int split_min,
-                            unsigned* __restrict__ keys, int* __restrict__ vals, int* status) {
+                            unsigned* __restrict__ keys, int* __restrict__ vals, int* status, const IbZeroed z) {
+  // the words that the kernels after this one count in start from zero
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < z.nranges; i += gridDim.x * blockDim.x) z.ranges[i] = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < z.ncounters; i += gridDim.x * blockDim.x) z.counters[i] = 0;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < z.ntickets) z.tickets[threadIdx.x] = 0;
+    if (threadIdx.x < 2 * z.redo_groups) z.redo[(threadIdx.x >> 1) * z.redo_stride + (threadIdx.x & 1)] = 0;
+  }
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
     int s[4], l[4], st[4] = {0, 0, 0, 0};
     bool bad = false;
@@ -241,6 +248,7 @@ __global__ void ib_classify(const int* __restrict__ quartets, const int* __restr
     }
     keys[q] = (unsigned(skip) << 15) | (unsigned(gen) << 14) | (unsigned(fp32) << 13) | low;
     vals[q] = q;
+    z.flags[q] = 0;
   }
 }
 
@@ -293,6 +301,9 @@ __global__ void ib_build_items(const unsigned* __restrict__ keys, const int* __r
     const int rs = 2 * (cid + fp32 * IB_NCLASS);
     if (prev != slot) ranges[rs] = p;
     if (next != slot) ranges[rs + 1] = p + 1;
+    // key bits 0-3: 15 - log2 of the primitive quartet count, ascending in a class
+    const unsigned lim = 15 - IB_MERGED_LONG_LOG2;
+    if (!fp32 && (key & 15u) <= lim && (next != slot || (keys[p + 1] & 15u) > lim)) ranges[IB_SLOT_LONG_END + cid] = p + 1;
   }
 }
 
@@ -456,10 +467,9 @@ __global__ void ib_diag_max(const int* __restrict__ pairs, int n, const int* __r
   }
 }
 
-// Apply 4 spherical (or truncating) transforms index by index and emit the
-// caller-ordered compact block: res[blk][ia + na*(ib + nb*(ic + nc*id))].
-// One block per contraction combination; T[i] == nullptr keeps the first n[i]
-// Cartesian components.
+// Apply 4 spherical transforms index by index and emit the caller-ordered
+// compact block: res[blk][ia + na*(ib + nb*(ic + nc*id))].  One block per
+// contraction combination.
 struct IbXform {
   const double* T[4];
   int l[4], n[4];
@@ -486,13 +496,8 @@ __global__ void ib_transform_blocks(const IbXform x, const double* __restrict__ 
     for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
       const int in = idx % inner, rest = idx / inner;
       const int s = rest % nout, o = rest / nout;
-      double v;
-      if (x.T[axis]) {
-        v = 0.0;
-        for (int c = 0; c < nin; ++c) v += x.T[axis][c + s * nin] * src[((size_t)o * nin + c) * inner + in];
-      } else {
-        v = src[((size_t)o * nin + s) * inner + in];
-      }
+      double v = 0.0;
+      for (int c = 0; c < nin; ++c) v += x.T[axis][c + s * nin] * src[((size_t)o * nin + c) * inner + in];
       dst[idx] = v;
     }
     __syncthreads();
@@ -517,6 +522,20 @@ int packed_sph_size() {
   int n = 0;
   for (int l = 0; l <= IB_LMAX; ++l) n += ncart_h(l) * (2 * l + 1);
   return n;
+}
+
+// Largest l of class cid (pair ids pb >= pk, ib_pair_ext; IB_NPAIR is (2,3)).
+int class_lmax(int cid) {
+  int pb = 0;
+  while ((pb + 1) * (pb + 2) / 2 <= cid) ++pb;
+  const int pk = cid - pb * (pb + 1) / 2;
+  auto pair_lmax = [](int p) {
+    if (p == IB_NPAIR) return 3;
+    int la = 0;
+    while ((la + 1) * (la + 2) / 2 <= p) ++la;
+    return la;
+  };
+  return std::max(pair_lmax(pb), pair_lmax(pk));
 }
 
 int get_context(Context** out) {
@@ -561,6 +580,12 @@ int get_context(Context** out) {
     IB_CUDA(c->counters.ensure((kNCounters + 1) * sizeof(int)));  // + the drop-in's own
     IB_CUDA(c->status.ensure(sizeof(int)));
     IB_CUDA(cudaMemset(c->status.p, 0, sizeof(int)));
+    IB_CUDA(c->tickets.ensure(kTickets * sizeof(int)));
+    IB_CUDA(c->small_ctl.ensure((18 + 2 * (size_t)kSmallBatch) * sizeof(int)));
+    IB_CUDA(c->small_items.ensure((size_t)kSmallBatch * sizeof(IbItem)));
+    c->last_status = c->status.as<int>();
+    IB_CUDA(ib_small_prepare_cart());
+    IB_CUDA(ib_small_prepare_sph());
     ib_register_emitted_classes(c->table);
     std::vector<int> kind(IB_NCLASS, 0);
     for (int cid = 0; cid < IB_NCLASS; ++cid) {
@@ -570,6 +595,11 @@ int get_context(Context** out) {
       for (int v = 0; v < 4 * IB_NMINB; ++v) c->occ[cid][v] = std::max(1, c->table[cid].occupancy(v));
       for (int v = 0; v < 4; ++v) c->minb_idx[cid][v] = std::min(std::max(ib_tuned_minb[cid][v], 0), IB_NMINB - 1);
       c->slice_cap[cid] = ib_tuned_slice_cap[cid];
+    }
+    for (int cid = IB_NCLASS - 1; cid >= 0; --cid) {
+      if (!c->table[cid].launch) continue;
+      c->classes.push_back(cid);
+      c->lmax_of.push_back(class_lmax(cid));
     }
     if (const char* env = std::getenv("INTCEPTION_B200_SLICE_BOOST")) c->slice_boost = std::max(1, std::atoi(env));
     if (const char* env = std::getenv("INTCEPTION_B200_MAX_SLICES"))
@@ -609,20 +639,6 @@ long long generic_slice(int lmax) {
   return (best + 31) / 32 * 32;
 }
 
-// Largest l of class cid (pair ids pb >= pk, ib_pair_ext; IB_NPAIR is (2,3)).
-int class_lmax(int cid) {
-  int pb = 0;
-  while ((pb + 1) * (pb + 2) / 2 <= cid) ++pb;
-  const int pk = cid - pb * (pb + 1) / 2;
-  auto pair_lmax = [](int p) {
-    if (p == IB_NPAIR) return 3;
-    int la = 0;
-    while ((la + 1) * (la + 2) / 2 <= p) ++la;
-    return la;
-  };
-  return std::max(pair_lmax(pb), pair_lmax(pk));
-}
-
 // The generic kernel over the redo list of a (on stream s, after the class
 // kernels that fill it); tickets: a zeroed pair (null: fixed order, no cluster).
 cudaError_t redo_launch(Context* c, cudaStream_t s, const IbLaunch& a, bool sph, int lmax, int* tickets) {
@@ -638,20 +654,41 @@ cudaError_t redo_launch(Context* c, cudaStream_t s, const IbLaunch& a, bool sph,
 
 // Launch the emitted kernels for the given variants and the generic kernel;
 // items/ranges already on the device.  Returns the number of kernels launched.
-int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, bool fp64_present, bool fp32_present, bool sph,
+int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, int nq, bool fp64_present, bool fp32_present, bool sph,
              int lmax, int* nlaunch, const ZeroFill* zf = nullptr) {
-  // the generic kernel's tickets: pair 0 for its range launch, pair 1 + g for redo list g
-  IB_CUDA(c->tickets.ensure(kTickets * sizeof(int)));
-  IB_CUDA(cudaMemsetAsync(c->tickets.p, 0, kTickets * sizeof(int), s));
+  // the generic kernel's tickets (zeroed by classify): pair 0 for its range launch, pair 1 + g for redo list g
   int* const tk = c->tickets.as<int>();
+  // side streams: one per launch, up to nside (an l <= 2 batch needs 22 of the 40)
+  // few l <= 2 quartets: the class kernels as one kernel on the caller's stream
+  // (with the HRR check on no quartet is routed to the generic kernel)
+  if (nq <= kMergedBatch && lmax == ib_lmax_emitted && !fp32_present && a.redo && a.hrr_tol > 0.0) {
+    if (zf) {
+      ib_zero_screened<<<std::min(c->nsm * 4, (nq + 255) / 256), 256, 0, s>>>(zf->keys, zf->nq, zf->quartets,
+                                                                              zf->shell_l, zf->out_off, sph ? 1 : 0, a.out);
+      ++*nlaunch;
+    }
+    IbLaunch am = a;
+    am.counter = c->counters.as<int>();
+    const int grid = std::min(2 * c->nsm, nq);
+    IB_CUDA(sph ? ib_merged_launch_sph(grid, s, am) : ib_merged_launch_cart(grid, s, am));
+    IB_CUDA(redo_launch(c, s, a, sph, lmax, tk + 2));
+    *nlaunch += 2;
+    return IB_OK;
+  }
+  const bool generic = (lmax > ib_lmax_emitted || lmax >= 2) && fp64_present;
+  int nuse = (generic ? 1 : 0) + (zf ? 1 : 0);
+  for (size_t i = 0; i < c->classes.size(); ++i)
+    if (c->lmax_of[i] <= lmax)
+      nuse += (fp64_present ? 1 : 0) + (fp32_present && c->kind_h[c->classes[i]] == 2 ? 2 : 0);
+  nuse = std::max(1, std::min(nuse, c->nside));
   IB_CUDA(cudaEventRecord(c->fork, s));
-  for (int i = 0; i < c->nside; ++i) IB_CUDA(cudaStreamWaitEvent(c->side[i], c->fork, 0));
+  for (int i = 0; i < nuse; ++i) IB_CUDA(cudaStreamWaitEvent(c->side[i], c->fork, 0));
   int k = 0;
   // redo lists: one per group of side streams when the batch has several
   // (the class kernels of side stream j fill list j mod G; each group's redo
   // launch follows its own class kernels and overlaps the others')
   const bool redo_on = a.redo && a.hrr_tol > 0.0;
-  const int G = redo_on ? std::min(c->redo_groups, c->nside) : 1;
+  const int G = redo_on ? std::min(c->redo_groups, nuse) : 1;
   // generic-kernel scratch: the range launch's region, then one per grouped redo launch
   const long long gslice = generic_slice(lmax);
   const long long gfull = std::max<long long>(
@@ -662,7 +699,7 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, bool fp64_present, b
   // first with 4 blocks per SM: measured no slower than 1 or 2 blocks per SM, or
   // than launching it after the class kernels)
   if (zf) {
-    ib_zero_screened<<<c->nsm * 4, 256, 0, c->side[c->nside - 1]>>>(zf->keys, zf->nq, zf->quartets, zf->shell_l,
+    ib_zero_screened<<<c->nsm * 4, 256, 0, c->side[nuse - 1]>>>(zf->keys, zf->nq, zf->quartets, zf->shell_l,
                                                                      zf->out_off, sph ? 1 : 0, a.out);
     ++*nlaunch;
   }
@@ -674,13 +711,12 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, bool fp64_present, b
     cudaError_t e = c->scratch.ensure((size_t)(gfull + (G > 1 ? G * ggroup : 0)) * gslice * sizeof(double));
     if (e != cudaSuccess) return e;
     // heavy quartets of the range over clusters too (INTCEPTION_B200_GENERIC_SPLIT 2)
-    e = ib_generic_launch((int)gfull, c->side[k % c->nside], a,
+    e = ib_generic_launch((int)gfull, c->side[k % nuse], a,
                           IbGenWork{kSlotGenHeavy, kSlotGenLight, 0, tk, ib_generic_split() >= 2 ? kSplitRange : 0},
                           sph ? 1 : 0, c->scratch.as<double>(), gslice);
     ++k;
     return e;
   };
-  const bool generic = (lmax > ib_lmax_emitted || lmax >= 2) && fp64_present;
   if (generic && lmax >= 3) IB_CUDA(launch_generic());
   for (int prec = 0; prec < 2; ++prec) {
     if ((prec == 0 && !fp64_present) || (prec == 1 && !fp32_present)) continue;
@@ -688,13 +724,14 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, bool fp64_present, b
     if (prec == 1) ap.ranges = a.ranges + kSlotFp32;
     const int variant = prec * 2 + (sph ? 1 : 0);
     // heaviest classes first so they start early on their streams
-    for (int cid = IB_NCLASS - 1; cid >= 0; --cid) {
-      if (!c->table[cid].launch || class_lmax(cid) > lmax) continue;  // no quartet of the batch has this class
+    for (size_t ci = 0; ci < c->classes.size(); ++ci) {
+      const int cid = c->classes[ci];
+      if (c->lmax_of[ci] > lmax) continue;  // no quartet of the batch has this class
       if (prec == 1 && c->kind_h[cid] != 2) continue;
       const int vt = variant + 4 * c->minb_idx[cid][variant];
       const int grid = c->nsm * c->occ[cid][vt];
-      cudaStream_t ss = c->side[k % c->nside];
-      if (G > 1) ap.redo = a.redo + (size_t)((k % c->nside) % G) * c->redo_stride;
+      cudaStream_t ss = c->side[k % nuse];
+      if (G > 1) ap.redo = a.redo + (size_t)((k % nuse) % G) * c->redo_stride;
       ap.max_slices = c->slice_cap[cid];
       ap.counter = c->counters.as<int>() + prec * IB_NCLASS + cid;
       c->table[cid].launch(vt, grid, ss, ap);
@@ -716,9 +753,9 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, bool fp64_present, b
   IB_CUDA(cudaGetLastError());
   if (G > 1) {
     // group g's redo on side stream g, after every class kernel of its streams
-    for (int j = 0; j < c->nside; ++j) IB_CUDA(cudaEventRecord(c->join[j], c->side[j]));
+    for (int j = 0; j < nuse; ++j) IB_CUDA(cudaEventRecord(c->join[j], c->side[j]));
     for (int g = 0; g < G; ++g) {
-      for (int j = g; j < c->nside; j += G)
+      for (int j = g; j < nuse; j += G)
         if (j != g) IB_CUDA(cudaStreamWaitEvent(c->side[g], c->join[j], 0));
       IbLaunch ag = a;
       ag.redo = a.redo + (size_t)g * c->redo_stride;
@@ -728,7 +765,7 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, bool fp64_present, b
       ++k;
     }
   }
-  for (int i = 0; i < c->nside; ++i) {
+  for (int i = 0; i < nuse; ++i) {
     IB_CUDA(cudaEventRecord(c->join[i], c->side[i]));
     IB_CUDA(cudaStreamWaitEvent(s, c->join[i], 0));
   }
@@ -800,8 +837,14 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
     o_T[i] = cur;
     cur = al(cur + tsize[i] * sizeof(double));
   }
-  const size_t total = cur;
-  IB_CUDA(c->h_stage.ensure(total));
+  // control words that the kernels count in, zero in the staged block: quartet
+  // counter [0], redo counts [2, 3] with the list's slots and flags after them
+  const size_t o_ctl = cur;
+  cur = al(cur + (4 + 2 * (size_t)nblk) * sizeof(int));
+  // behind the staged block: the status word (zero too), then the result
+  const size_t o_status = cur, staged = cur + 256, o_res = staged;
+  const size_t total = o_res + (size_t)nblk * res_block * sizeof(double);
+  IB_CUDA(c->h_stage.ensure(staged));
   IB_CUDA(c->d_stage.ensure(total));
   char* h = static_cast<char*>(c->h_stage.p);
   int* hl = reinterpret_cast<int*>(h + o_l);
@@ -900,12 +943,18 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
   }
   for (int i = 0; i < 4; ++i)
     if (sph) std::memcpy(h + o_T[i], sh[i].T, tsize[i] * sizeof(double));
-  IB_CUDA(c->d_cart.ensure((size_t)nblk * cart_block * sizeof(double)));
-  IB_CUDA(c->d_res.ensure((size_t)nblk * (res_block + 2 * cart_block) * sizeof(double)));
-  IB_CUDA(c->h_res.ensure((size_t)nblk * res_block * sizeof(double)));
+  // Cartesian blocks need no transform: the kernels write the result itself
+  if (sph) {
+    IB_CUDA(c->d_cart.ensure((size_t)nblk * cart_block * sizeof(double)));
+    IB_CUDA(c->d_res.ensure((size_t)nblk * 2 * cart_block * sizeof(double)));
+  }
+  IB_CUDA(c->h_res.ensure(total - o_ctl));
+  std::memset(h + o_ctl, 0, staged - o_ctl);
   cudaStream_t s = c->stream;
   char* d = static_cast<char*>(c->d_stage.p);
-  IB_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, s));
+  IB_CUDA(cudaMemcpyAsync(d, h, staged, cudaMemcpyHostToDevice, s));
+  double* dres = reinterpret_cast<double*>(d + o_res);
+  int* dctl = reinterpret_cast<int*>(d + o_ctl);
   IbLaunch a = base_launch(c);
   a.items = reinterpret_cast<const IbItem*>(d + o_it);
   a.ranges = reinterpret_cast<const int*>(d + o_rg);
@@ -915,26 +964,22 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
   a.shell_xyz = reinterpret_cast<const double*>(d + o_xyz);
   a.prim_exp = reinterpret_cast<const double*>(d + o_e);
   a.prim_coef = reinterpret_cast<const double*>(d + o_c);
-  a.out = c->d_cart.as<double>();
-  IB_CUDA(cudaMemsetAsync(c->status.p, 0, sizeof(int), s));
+  a.out = sph ? c->d_cart.as<double>() : dres;
+  a.status = reinterpret_cast<int*>(d + o_status);
+  c->last_status = c->last_redo = nullptr;  // read from the host copies below
+  c->host_status = c->host_redo = 0;
+  c->flags_nq = 0;
   if (emitted) {
     const int vt = 4 * c->minb_idx[cidx][0];
-    const int grid = std::max(1, std::min(c->nsm * c->occ[cidx][vt], (nblk + IB_BLOCK - 1) / IB_BLOCK));
-    a.counter = c->counters.as<int>() + kNCounters;  // never used by a batch that may still run
-    IB_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(int), s));
-    IB_CUDA(c->flags.ensure((size_t)nblk * sizeof(int)));
-    IB_CUDA(cudaMemsetAsync(c->flags.p, 0, (size_t)nblk * sizeof(int), s));
-    IB_CUDA(c->redo.ensure((size_t)(nblk + 2) * sizeof(int)));
-    IB_CUDA(cudaMemsetAsync(c->redo.p, 0, 2 * sizeof(int), s));
-    c->redo_groups = 1;
-    c->redo_stride = nblk + 2;
-    c->flags_nq = nblk;
-    a.flags = c->flags.as<int>();
-    a.redo = c->redo.as<int>();
+    const int grid = std::max(1, std::min(c->nsm * c->occ[cidx][vt], nblk));
+    a.counter = dctl;
+    a.redo = dctl + 2;
+    a.flags = dctl + 4 + nblk;
     a.redo_cap = nblk;
     a.hrr_tol = c->hrr_tol;
     c->table[cidx].launch(vt, grid, s, a);
-    if (a.hrr_tol > 0.0)
+    // a class without an HRR has no check that could fill the list
+    if (a.hrr_tol > 0.0 && (lperm[1] > 0 || lperm[3] > 0))
       IB_CUDA(redo_launch(c, s, a, false, std::max(std::max(sh[0].l, sh[1].l), std::max(sh[2].l, sh[3].l)),
                           nullptr));
   } else {
@@ -947,26 +992,30 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
                               slice));
   }
   IB_CUDA(cudaGetLastError());
-  IbXform x;
-  for (int i = 0; i < 4; ++i) {
-    x.T[i] = sph ? reinterpret_cast<const double*>(d + o_T[i]) : nullptr;
-    x.l[i] = sh[i].l;
-    x.n[i] = sh[i].n;
+  if (sph) {
+    IbXform x;
+    for (int i = 0; i < 4; ++i) {
+      x.T[i] = reinterpret_cast<const double*>(d + o_T[i]);
+      x.l[i] = sh[i].l;
+      x.n[i] = sh[i].n;
+    }
+    x.nblk = nblk;
+    x.cart_block = cart_block;
+    x.res_block = res_block;
+    ib_transform_blocks<<<nblk, 128, 0, s>>>(x, c->d_cart.as<double>(), dres, c->d_res.as<double>());
+    IB_CUDA(cudaGetLastError());
   }
-  x.nblk = nblk;
-  x.cart_block = cart_block;
-  x.res_block = res_block;
-  double* dres = c->d_res.as<double>();
-  ib_transform_blocks<<<nblk, 128, 0, s>>>(x, c->d_cart.as<double>(), dres, dres + (size_t)nblk * res_block);
-  IB_CUDA(cudaGetLastError());
-  int hstatus = 0;
-  IB_CUDA(cudaMemcpyAsync(c->h_res.p, dres, (size_t)nblk * res_block * sizeof(double), cudaMemcpyDeviceToHost, s));
-  IB_CUDA(cudaMemcpyAsync(&hstatus, c->status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  // control words, status word and result in one copy
+  IB_CUDA(cudaMemcpyAsync(c->h_res.p, d + o_ctl, total - o_ctl, cudaMemcpyDeviceToHost, s));
   IB_CUDA(cudaStreamSynchronize(s));
+  const char* hr = static_cast<const char*>(c->h_res.p);
+  const int hstatus = *reinterpret_cast<const int*>(hr + (o_status - o_ctl));
+  c->host_status = hstatus;
+  c->host_redo = reinterpret_cast<const int*>(hr)[2] + reinterpret_cast<const int*>(hr)[3];
   if (hstatus) return set_status(hstatus, "device kernel reported status " + std::to_string(hstatus));
   // place the compact result at the caller's strides (the emitted code's final
   // copy loop, contracted_general.py:1808-1876)
-  const double* r = static_cast<const double*>(c->h_res.p);
+  const double* r = reinterpret_cast<const double*>(hr + (o_res - o_ctl));
   b = 0;
   for (int ka = 0; ka < sh[0].ncont; ++ka)
     for (int kb = 0; kb < sh[1].ncont; ++kb)
@@ -1089,6 +1138,45 @@ int resolve_stream(Context* c, void* stream, cudaStream_t* s) {
   return IB_OK;
 }
 
+// A small l <= 2 FP64 batch (kSmallBatch): one kernel in the caller's order,
+// then the redo list's.
+int small_batch(Context* c, const intception_b200_basis* basis, const int* quartets, const long long* out_off, int nq,
+                int spherical, const double* bounds, double skip_below, double* out, cudaStream_t s, int* nl,
+                bool screen_prims) {
+  // words zeroed by one memset: status [0], tickets [2, 3], flags [16, 16 + nq),
+  // the redo list's counts; its slots follow
+  int* ctl = c->small_ctl.as<int>();
+  IB_CUDA(cudaMemsetAsync(ctl, 0, (18 + (size_t)nq) * sizeof(int), s));
+  IbLaunch a = base_launch(c);
+  a.items = c->small_items.as<IbItem>();
+  a.shell_l = basis->shell_l;
+  a.shell_k = basis->shell_k;
+  a.shell_ptr = basis->shell_ptr;
+  a.shell_xyz = basis->shell_xyz;
+  a.prim_exp = basis->prim_exp;
+  a.prim_coef = basis->prim_coef;
+  a.out = out;
+  a.prim_tol = screen_prims ? c->prim_tol : 0.0;
+  a.status = ctl;
+  a.flags = ctl + 16;
+  a.redo = ctl + 16 + nq;
+  a.redo_cap = nq;
+  a.hrr_tol = c->hrr_tol;
+  c->last_status = ctl;
+  c->last_redo = a.redo;
+  c->redo_groups = 1;
+  c->flags_nq = 0;
+  const IbSmallArgs b = {quartets, out_off, bounds, skip_below, c->small_items.as<IbItem>(), nq, basis->lmax};
+  const int grid = std::min(2 * c->nsm, nq);
+  IB_CUDA(spherical ? ib_small_launch_sph(grid, s, a, b) : ib_small_launch_cart(grid, s, a, b));
+  ++*nl;
+  if (a.hrr_tol > 0.0) {
+    IB_CUDA(redo_launch(c, s, a, spherical != 0, basis->lmax, ctl + 2));
+    ++*nl;
+  }
+  return set_status(IB_OK, "");
+}
+
 // The batch pipeline on stream s; the caller holds the context lock.
 int batch_impl(Context* c, const intception_b200_basis* basis, const int* quartets, const long long* out_off, int nq,
                int spherical, int precision, const double* bounds, double skip_below, double fp32_below,
@@ -1100,6 +1188,9 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   if ((precision == IB_PREC_MIXED || skip_below > 0.0) && !bounds)
     return set_status(IB_ERR_ARG, "eri_batch: mixed precision and screening need bounds");
   if (nq == 0) return set_status(IB_OK, "");
+  if (nq <= kSmallBatch && basis->lmax <= ib_lmax_emitted && precision == IB_PREC_FP64 && c->hrr_tol > 0.0)
+    return small_batch(c, basis, quartets, out_off, nq, spherical, skip_below > 0.0 ? bounds : nullptr, skip_below, out,
+                       s, nl, screen_prims);
   IB_CUDA(c->keys.ensure((size_t)nq * sizeof(unsigned)));
   IB_CUDA(c->keys2.ensure((size_t)nq * sizeof(unsigned)));
   IB_CUDA(c->vals.ensure((size_t)nq * sizeof(int)));
@@ -1109,9 +1200,17 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   IB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, c->keys.as<unsigned>(), c->keys2.as<unsigned>(),
                                           c->vals.as<int>(), c->vals2.as<int>(), nq, 0, kKeyBits, s));
   IB_CUDA(c->cub_tmp.ensure(tmp_bytes));
-  IB_CUDA(cudaMemsetAsync(c->ranges.p, 0, kNRanges * sizeof(int), s));
-  IB_CUDA(cudaMemsetAsync(c->counters.p, 0, kNCounters * sizeof(int), s));
+  IB_CUDA(c->flags.ensure((size_t)nq * sizeof(int)));
+  // l >= 3 batches: four redo lists, one per group of side streams (dispatch)
+  c->redo_groups = (basis->lmax >= 3 && c->hrr_tol > 0.0) ? kRedoGroups : 1;
+  c->redo_stride = nq + 2;
+  IB_CUDA(c->redo.ensure((size_t)c->redo_groups * (nq + 2) * sizeof(int)));
+  c->flags_nq = nq;
+  c->last_status = c->status.as<int>();
+  c->last_redo = c->redo.as<int>();
   IB_CUDA(cudaMemsetAsync(c->status.p, 0, sizeof(int), s));
+  const IbZeroed zeroed = {c->ranges.as<int>(), c->counters.as<int>(), c->tickets.as<int>(), c->redo.as<int>(),
+                           c->flags.as<int>(), kNRanges, kNCounters, kTickets, c->redo_groups, c->redo_stride};
   const int grid = std::min((nq + 255) / 256, c->nsm * 16);
   const bool use_bounds = bounds != nullptr && (precision == IB_PREC_MIXED || skip_below > 0.0);
   ib_classify<<<grid, 256, 0, s>>>(quartets, basis->shell_l, basis->shell_k, basis->shell_ptr, basis->prim_exp,
@@ -1119,7 +1218,7 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
                                    use_bounds ? bounds : nullptr, skip_below, fp32_below,
                                    precision == IB_PREC_MIXED ? 1 : 0, c->kind.as<int>(), c->hrr_tol > 0.0 ? 0 : 1,
                                    ib_generic_split_min(), c->keys.as<unsigned>(),
-                                   c->vals.as<int>(), c->status.as<int>());
+                                   c->vals.as<int>(), c->status.as<int>(), zeroed);
   ++*nl;
   IB_CUDA(cudaGetLastError());
   IB_CUDA(cub::DeviceRadixSort::SortPairs(c->cub_tmp.p, tmp_bytes, c->keys.as<unsigned>(), c->keys2.as<unsigned>(),
@@ -1141,22 +1240,13 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   a.prim_coef = basis->prim_coef;
   a.out = out;
   a.prim_tol = screen_prims ? c->prim_tol : 0.0;
-  IB_CUDA(c->flags.ensure((size_t)nq * sizeof(int)));
-  IB_CUDA(cudaMemsetAsync(c->flags.p, 0, (size_t)nq * sizeof(int), s));
-  // l >= 3 batches: four redo lists, one per group of side streams (dispatch)
-  c->redo_groups = (basis->lmax >= 3 && c->hrr_tol > 0.0) ? kRedoGroups : 1;
-  c->redo_stride = nq + 2;
-  IB_CUDA(c->redo.ensure((size_t)c->redo_groups * (nq + 2) * sizeof(int)));
-  for (int g = 0; g < c->redo_groups; ++g)
-    IB_CUDA(cudaMemsetAsync(c->redo.as<int>() + (size_t)g * (nq + 2), 0, 2 * sizeof(int), s));
-  c->flags_nq = nq;
   a.flags = c->flags.as<int>();
   a.redo = c->redo.as<int>();
   a.redo_cap = nq;
   a.hrr_tol = c->hrr_tol;
   if (precision == IB_PREC_MIXED) a.mixed_tol = mixed_tol;
   const ZeroFill zf = {c->keys.as<unsigned>(), nq, quartets, basis->shell_l, out_off};
-  return dispatch(c, s, a, true, precision == IB_PREC_MIXED, spherical != 0, basis->lmax, nl,
+  return dispatch(c, s, a, nq, true, precision == IB_PREC_MIXED, spherical != 0, basis->lmax, nl,
                   use_bounds && skip_below > 0.0 ? &zf : nullptr);
 }
 }  // namespace
@@ -1461,12 +1551,12 @@ int intception_b200_last_fp32_rejections(void) {
 int intception_b200_last_hrr_redo(void) {
   Context* c = nullptr;
   if (get_context(&c)) return -1;
-  if (!c->redo.p) return 0;
+  if (!c->last_redo) return c->host_redo;
   IB_CUDA(cudaDeviceSynchronize());
   int total = 0;
   for (int g = 0; g < c->redo_groups; ++g) {
     int h[2] = {0, 0};  // heavy and light counts
-    IB_CUDA(cudaMemcpy(h, c->redo.as<int>() + (size_t)g * c->redo_stride, 2 * sizeof(int), cudaMemcpyDeviceToHost));
+    IB_CUDA(cudaMemcpy(h, c->last_redo + (size_t)g * c->redo_stride, 2 * sizeof(int), cudaMemcpyDeviceToHost));
     total += h[0] + h[1];
   }
   return total;
@@ -1554,7 +1644,8 @@ int intception_b200_batch_status(void) {
   if (st) return st;
   int h = 0;
   IB_CUDA(cudaDeviceSynchronize());
-  IB_CUDA(cudaMemcpy(&h, c->status.p, sizeof(int), cudaMemcpyDeviceToHost));
+  if (!c->last_status) return c->host_status;
+  IB_CUDA(cudaMemcpy(&h, c->last_status, sizeof(int), cudaMemcpyDeviceToHost));
   return h;
 }
 

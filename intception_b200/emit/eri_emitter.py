@@ -410,7 +410,7 @@ def thread_class(c):
     return c[2] + c[3] == 0 or n <= THREAD_TARGETS
 
 
-THREAD_TARGETS = 60
+THREAD_TARGETS = 54
 
 
 def fp64_emitter(c):
@@ -465,6 +465,39 @@ def class_source(c, fp32):
     return '\n'.join(parts), dict(kind=e.kind, G=e.G, budget=e.budget())
 
 
+def emit_small(outdir):
+    """The small-batch kernel: every l <= LMAX_EMIT class in one kernel (a
+    translation unit per output kind)."""
+    es = [fp64_emitter(c) for c in canonical_classes(LMAX_EMIT)]
+    for e in es:
+        e.quartet_code()
+    stride = max(e.per_group for e in es)  # slots of different classes lie side by side
+    smem = 8 * 4 * stride
+    for sph in (0, 1):
+        T = 'true' if sph else 'false'
+        src = ['// Generated by intception_b200/emit/eri_emitter.py -- do not edit.', '#include "ib_small.cuh"', '']
+        src += [e.function(stride) for e in es]
+        src += ['struct IbSmallSwitch_%s {' % ('sph' if sph else 'cart'),
+                '  static constexpr int NC = %d;  // classes, in descending order' % len(es),
+                '  static __device__ __forceinline__ int cid(int k) {',
+                '    constexpr short ids[NC] = {%s};' % ', '.join(str(e.cid) for e in reversed(es)),
+                '    return ids[k];',
+                '  }',
+                '  static __device__ __forceinline__ void run(const IbLaunch& a, const IbItem* it, int p, int W, int cid) {',
+                '    switch (cid) {']
+        src += ['      case %d: %s_one<%s>(a, it, p, W); break;' % (e.cid, e.name, T) for e in es]
+        src += ['    }', '  }', '};',
+                'cudaError_t ib_small_prepare_%s() { return ib_small_prepare<IbSmallSwitch_%s, %s>(%d); }'
+                % ('sph' if sph else 'cart', 'sph' if sph else 'cart', T, smem),
+                'cudaError_t ib_small_launch_%s(int grid, cudaStream_t s, const IbLaunch& a, const IbSmallArgs& b) {'
+                % ('sph' if sph else 'cart'),
+                '  return ib_small_go<IbSmallSwitch_%s, %s>(grid, %d, s, a, b);'
+                % ('sph' if sph else 'cart', T, smem), '}',
+                'cudaError_t ib_merged_launch_%s(int grid, cudaStream_t s, const IbLaunch& a) {' % ('sph' if sph else 'cart'),
+                '  return ib_merged_go<IbSmallSwitch_%s, %s>(grid, %d, s, a);' % ('sph' if sph else 'cart', T, smem), '}']
+        _write_if_changed(os.path.join(outdir, 'eri_small_%s.cu' % ('sph' if sph else 'cart')), '\n'.join(src) + '\n')
+
+
 def emit_all(outdir, lmax=LMAX_EMIT, ngroups=24):
     """Write the class translation units and the dispatch table into outdir.
     Returns the list of per-class statistics."""
@@ -510,6 +543,7 @@ def emit_all(outdir, lmax=LMAX_EMIT, ngroups=24):
     for g in range(ngroups):
         disp.append('  ib_register_group_%d(table);' % g)
     disp.append('}')
+    emit_small(outdir)
     # autotuned defaults (intception_b200/tuning.json, written by
     # python -m intception_b200.autotune on a GPU): per class and variant the
     # register-budget index, per class the slice cap and whether the FP32 tier

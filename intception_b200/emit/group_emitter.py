@@ -712,7 +712,7 @@ class GroupEmitter:
         src.append('  for (int p = %s; p < end; p = %s) {' % (grab, grab))
         src.append('    if (sizeof(R) == 8 && a.recheck && !(a.flags[p] & 1)) continue;  // uniform over the quartet\'s lanes')
         src.append('    IbQuartet g;')
-        src.append('    ib_load_quartet(a, p, g);')
+        src.append('    ib_load_quartet(a, a.items[p], g);')
         src.append('    const int kb_ = g.k[1], kd_ = g.k[3];')
         src.append('    const int kab = g.k[0] * kb_, kcd = g.k[2] * kd_;')
         # primitive screening (a.prim_tol > 0) for quartets of one pair tile a

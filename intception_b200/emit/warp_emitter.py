@@ -80,8 +80,12 @@ class WarpEmitter(GroupEmitter):
     def name(self):
         return 'ib_%s_%s' % (self.kind, self.tag)
 
-    def kernel(self):
-        """CUDA source of the class's FP64 kernel."""
+    def quartet_code(self, stride=None):
+        """Code of one quartet (item *itp, sorted index p) on its lanes: the
+        declarations that depend on the lane only, and the evaluation.
+        stride: doubles of shared memory between groups (default: the class's
+        own need; a kernel of several classes gives them one stride, as their
+        groups lie side by side)."""
         G = self.G
         # threads per block: four warps, or one group where that is not a part of them
         self.block = 128 if G in (32, 64, 128) else G
@@ -101,21 +105,14 @@ class WarpEmitter(GroupEmitter):
         per_group = o_que + 2 * CHUNK // 4 + 2
         per_group += per_group & 1
         self.smem = 8 * (self.block // G) * per_group
+        self.per_group = per_group
+        if stride is not None:
+            assert stride >= per_group
+            per_group = stride
         NB = getattr(self, 'NB', 1)
         sync = 'ib_group_bar(gid, %d)' % G if wide else '__syncwarp()'
         src = []
         A = src.append
-        A('// ---- class (%d%d|%d%d): %s' % (self.la, self.lb, self.lc, self.ld, self.describe()))
-        src += self.constants()
-        A('template <bool SPH, int MINB>')
-        A('__global__ void __launch_bounds__(%d, MINB) %s(const IbLaunch a) {' % (self.block, self.name))
-        A('  extern __shared__ double ib_smem[];')
-        A('  constexpr int GPB = %d;  // groups per block' % (self.block // G))
-        A('  const int beg = a.ranges[2 * %d], end = a.ranges[2 * %d + 1];' % (self.cid, self.cid))
-        A('  const int W = ib_slices(end - beg, GPB, a.max_slices, a.slice_boost);')
-        A('  const int SPB = GPB / W;  // quartets in flight per block')
-        A('  if (beg + (int)blockIdx.x * SPB >= end) return;  // block-uniform')
-        A('  const int gid = threadIdx.x / %d, j = threadIdx.x %% %d;' % (G, G))
         A('  const unsigned sgmask = 0xffffffffu;')
         A('  const int sg = gid / W, w = gid - sg * W;  // quartet slot in the block, slice in the quartet')
         A('  const int SG = W * %d, r = w * %d + j;  // lanes per quartet, this lane among them' % (G, G))
@@ -128,11 +125,10 @@ class WarpEmitter(GroupEmitter):
             A('  int* __restrict__ qcnt = reinterpret_cast<int*>(sb + %d);' % (per_group - 2))
         A('  double* __restrict__ pd = sb0 + %d;' % o_pair)
         src += self.prologue()
-        grab = 'ib_grab(a.counter, beg, r, SG, sg, sgmask, 0, lcnt + 2)'
-        A('  for (int p = %s; p < end; p = %s) {' % (grab, grab))
-        A('    if (a.recheck && !(a.flags[p] & 1)) continue;  // uniform over the quartet\'s lanes')
+        head, src = src, []
+        A = src.append
         A('    IbQuartet g;')
-        A('    ib_load_quartet(a, p, g);')
+        A('    ib_load_quartet(a, *itp, g);')
         A('    const int kb_ = g.k[1], kd_ = g.k[3];')
         A('    const int kab = g.k[0] * kb_, kcd = g.k[2] * kd_;')
         # classes with a g shell build only the exact-zero lists: an earlier
@@ -236,10 +232,41 @@ class WarpEmitter(GroupEmitter):
         src += ['  ' + s for s in epi_cart]
         A('    }')
         A('    ib_sg_sync(SG, sg, sgmask);')
-        A('  }')
-        A('}')
-        A('')
-        return '\n'.join(src)
+        return head, src
+
+    def kernel(self):
+        """CUDA source of the class's FP64 kernel: its groups take the quartets
+        of the class's range one at a time."""
+        head, body = self.quartet_code()
+        src = ['// ---- class (%d%d|%d%d): %s' % (self.la, self.lb, self.lc, self.ld, self.describe())]
+        src += self.constants()
+        src += ['template <bool SPH, int MINB>',
+                '__global__ void __launch_bounds__(%d, MINB) %s(const IbLaunch a) {' % (self.block, self.name),
+                '  extern __shared__ double ib_smem[];',
+                '  constexpr int GPB = %d;  // groups per block' % (self.block // self.G),
+                '  const int beg = a.ranges[2 * %d], end = a.ranges[2 * %d + 1];' % (self.cid, self.cid),
+                '  const int W = ib_slices(end - beg, GPB, a.max_slices, a.slice_boost);',
+                '  const int SPB = GPB / W;  // quartets in flight per block',
+                '  if (beg + (int)blockIdx.x * SPB >= end) return;  // block-uniform',
+                '  const int gid = threadIdx.x / %d, j = threadIdx.x %% %d;' % (self.G, self.G)]
+        src += head
+        grab = 'ib_grab(a.counter, beg, r, SG, sg, sgmask, 0, lcnt + 2)'
+        src += ['  for (int p = %s; p < end; p = %s) {' % (grab, grab),
+                '    if (a.recheck && !(a.flags[p] & 1)) continue;  // uniform over the quartet\'s lanes',
+                '    const IbItem* __restrict__ itp = a.items + p;']
+        return '\n'.join(src + body + ['  }', '}', ''])
+
+    def function(self, stride):
+        """The same evaluation as a device function of one quartet, for the
+        small-batch kernel (G = 32: one to four warps a quartet)."""
+        assert self.G == 32
+        head, body = self.quartet_code(stride)
+        src = self.constants()
+        src += ['template <bool SPH>',
+                '__device__ __noinline__ void %s_one(const IbLaunch& a, const IbItem* itp, int p, int W) {' % self.name,
+                '  extern __shared__ double ib_smem[];',
+                '  const int gid = threadIdx.x / 32, j = threadIdx.x % 32;']
+        return '\n'.join(src + head + ['  (void)lcnt; (void)que;'] + body + ['}', ''])
 
     def split_bra(self):
         # measured as instructions of one warp: a whole bra recurrence per f

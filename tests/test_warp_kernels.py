@@ -1,0 +1,87 @@
+"""The warp-per-quartet kernels where their layout changes: batch sizes either
+side of the small-batch and merged-kernel limits, pair counts either side of the
+64-pair tile, and the Rys table's rows and range ends."""
+import numpy as np
+import pytest
+
+from conftest import tolerance
+from intception_b200 import basis, eri
+from intception_b200.emit import rys_table
+from oracle import loader
+
+
+@pytest.mark.parametrize('N', [2, 5, 9])
+def test_rys_rule_reproduces_boys_moments(N):
+    """sum_r w_r u_r^k = F_k(T), k < 2N, from the stored polynomials (first row,
+    one inside, the last) and from the rule beyond the table.  Table values are
+    rounded to double (2^-53 each) and u^k multiplies u's error by k."""
+    import mpmath as mp
+    mp.mp.dps = 60
+    last = rys_table.RYS_TMAX[N] * rys_table.RYS_H_INV - 1
+    checks = []
+    for row in (0, 17, last):
+        coef = rys_table._row(row)[N]
+        for x in (-1.0, -0.3, 0.999):
+            v = [sum(mp.mpf(c) * mp.mpf(x) ** k for k, c in enumerate(cs)) for cs in coef]
+            checks.append(((row + (mp.mpf(x) + 1) / 2) / rys_table.RYS_H_INV, v[0::2], v[1::2]))
+    for T in (mp.mpf(rys_table.RYS_TMAX[N]), mp.mpf(500)):
+        hw = rys_table._asymptotic(N)
+        checks.append((T, [h / T for h, _ in hw], [w / mp.sqrt(T) for _, w in hw]))
+    for T, u, w in checks:
+        F = rys_table._moments(T, 2 * N)
+        for k in range(2 * N):
+            s = sum(wr * ur ** k for ur, wr in zip(u, w))
+            assert abs(s / F[k] - 1) <= (2 * k + 4) * 2.0 ** -52, (N, T, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('sph', [False, True])
+@pytest.mark.parametrize('lmax', [1, 2])
+def test_batch_sizes_around_the_path_limits(sph, lmax):
+    """The first quartets of one list, evaluated in batches of 1, 296, 297, 3072
+    and 3073 quartets (small-batch kernel, merged kernel, one kernel per
+    class), unscreened and screened, against the oracle."""
+    import torch
+    b = basis.independent_quartet_batch(31, 3073, list(range(lmax + 1)), [1, 2, 3, 5], 0.1, 60.0, 6.0, sph)
+    head = b.subset(np.arange(300))
+    ref = loader.oracle_batch(head, basis.sph_matrices(6))
+    for nq in (1, 296, 297, 3072, 3073):
+        eng = eri.EriEngine(b.subset(np.arange(nq)))
+        n = int(head.out_off[min(nq, 300) - 1]) if nq < 300 else head.out_size
+        out = torch.full((eng.out_size,), 7.0, dtype=torch.float64, device='cuda')
+        eng.compute(out=out)
+        assert np.abs(out.cpu().numpy()[:n] - ref[:n]).max(initial=0.0) <= tolerance(ref), nq
+        bounds = eng.analytic_bounds()
+        out.fill_(7.0)
+        eri.set_prim_tol(1e-18)
+        eng.compute(out=out, bounds=bounds, skip_below=1e-9)
+        eri.set_prim_tol(0.0)
+        # a zeroed block is off by at most its bound, 5^4 dropped primitives by 1e-18 each
+        got, kept = out.cpu().numpy(), bounds.cpu().numpy() >= 1e-9
+        assert np.abs(got[:n] - ref[:n]).max(initial=0.0) <= 1e-9 + tolerance(ref)
+        assert (got != 7.0).all()
+        for q in np.nonzero(kept[:300])[0]:
+            o, m = int(head.out_off[q]), int(np.prod(head.block_dims(q)))
+            assert np.abs(got[o:o + m] - ref[o:o + m]).max() <= 625e-18 + tolerance(ref)
+        assert eng.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('ls', [(0, 0, 0, 0), (1, 0, 1, 0), (1, 1, 1, 1), (2, 1, 1, 1), (2, 2, 2, 1), (2, 2, 2, 2)])
+@pytest.mark.parametrize('ks', [(1, 1, 1, 1), (8, 8, 4, 8), (9, 8, 8, 8), (13, 11, 5, 13)])
+def test_pair_counts_around_the_tile(ls, ks):
+    """Pair counts 1, 64, 72 and 143 a side (one tile of pairs holds 64), with
+    and without primitive screening at 1e-18."""
+    rng = np.random.default_rng(7)
+    n = 3
+    sh = basis.make_shells(rng, np.tile(ls, n), np.tile(ks, n), 0.2, 8.0, 1.5)
+    q = np.arange(4 * n, dtype=np.int32).reshape(n, 4)
+    off, total = basis.packed_offsets(sh[0], q, True)
+    b = basis.ShellBatch(*sh, q, off, True, total)
+    ref = loader.oracle_batch(b, basis.sph_matrices(6))
+    eng = eri.EriEngine(b)
+    assert np.abs(eng.compute().cpu().numpy() - ref).max() <= tolerance(ref)
+    eri.set_prim_tol(1e-18)
+    out = eng.compute().cpu().numpy()
+    eri.set_prim_tol(0.0)
+    assert np.abs(out - ref).max() <= tolerance(ref) + np.prod(np.array(ks, float)) * 1e-18
