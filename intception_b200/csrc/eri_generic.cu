@@ -3,11 +3,12 @@
 // Used for the classes that have no unrolled kernel (some l > the emitted
 // maximum), for quartets whose pairs are best built on their lower-l shell,
 // and for the quartets the class kernels put on the redo list (HRR rounding
-// estimate over the tolerance).  Same schedule as the emitted kernels (HGP:
-// bra VRR, ket VRR with the electron-transfer term, contraction, bra HRR, ket
-// HRR, spherical transform), but every stage is a loop over the elements of
-// one recurrence level, spread over the block's threads, with the levels in
-// global scratch (one slice per resident block).  FP64 throughout.
+// estimate over the tolerance).  [e0|f0] by Rys quadrature as in the emitted
+// kernels (2D integrals of every root and axis in shared memory, products,
+// contraction), then bra HRR, ket HRR and spherical transform, every stage a
+// loop over its elements spread over the block's threads, with the contracted
+// table and the HRR layers in global scratch (one slice per resident block).
+// FP64 throughout.
 //
 // Each primitive pair is built on the shell that conditions its HRR
 // (ib_gen_orient): a contraction that mixes tight and diffuse exponents on
@@ -32,9 +33,13 @@
 //
 // Scratch slice layout (doubles), sizes from ib_generic_dims():
 //   acc  [nf * ne]                 contracted [e0|f0] stored [f][e], e in [la,la+lb], f in [lc,lc+ld]
-//   bra  [(L+2) * ncumE]           [e0|00]^(m) over every e <= la+lb
-//   ket  3 * klev                  [e0|f0]^(m) of the ket levels f >= 1, level f in slot f mod 3
 //   h0,h1 [hmax] ping-pong buffers for HRR and the spherical transform
+//
+// The products are what the kernel spends its time on: an item is one e with
+// one (f_x, f_y), so that I_x I_y is formed once for its (up to l_d + 1) f_z;
+// lanes run over e, whose 2D values are few and broadcast.  Vertical
+// recurrences with their levels in scratch did the same work with
+// (L+1)/2 times the elements, every one through L2.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -93,9 +98,6 @@ __device__ __forceinline__ int ib_gen_orient(int l0, int l1, double x0, double x
 struct IbGenShared {
   IbGenericDims d;
   double A[3], B[3], C[3], D[3], AB[3], CD[3];  // this pass's shell order
-  double PA[3], WP[3], QC[3], WQ[3];
-  double o2z, roz, o2e, roe, o2zpe;
-  double F[4 * IB_LMAX + 1];
   int k[4], ptr[4], st[4];     // this pass's shell order
   int s0[4], l0[4], st0[4];    // the item's shell order
   int use[2];                  // per pair: bit o set when some primitive pair has orientation o
@@ -130,6 +132,132 @@ __device__ __forceinline__ void ib_gen_tables(unsigned short* ct, unsigned short
 // nonzero exponent.
 __device__ __forceinline__ int ib_gen_dir(int x, int y) { return x > 0 ? 0 : (y > 0 ? 1 : 2); }
 
+// Products of the nb primitive quartets whose 2D tables are at tab: items
+// (e, f_x, f_y), lanes over e; NZ: the largest count of f_z.
+template <int NZ>
+__device__ __forceinline__ void ib_gen_products(int nb, int N, const IbGenericDims& d, double* __restrict__ acc,
+                                                const double* __restrict__ tab, const unsigned short* __restrict__ ct,
+                                                const unsigned char* __restrict__ cp) {
+  const int C1 = d.F + 1, TS = ((d.E + 1) * C1) | 1, npair = C1 * (C1 + 1) / 2;
+  for (int x = threadIdx.x; x < npair * d.ne; x += blockDim.x) {
+    const int q = x / d.ne, e = x - q * d.ne;
+    const int fx = cp[q] & 15, fy = cp[q] >> 4;  // x and y exponents, f_x + f_y <= F in this order for every F
+    const int z0 = max(0, d.lc - fx - fy), nz = d.F - fx - fy - z0 + 1;
+    int ex, ey, ez;
+    ib_ct_get(ct, d.e0 + e, ex, ey, ez);
+    const double* __restrict__ X = tab + ex * C1 + fx;
+    const double* __restrict__ Y = tab + TS + ey * C1 + fy;
+    const double* __restrict__ Z = tab + 2 * TS + ez * C1 + z0;
+    double v[NZ];
+#pragma unroll
+    for (int k = 0; k < NZ; ++k) v[k] = 0.0;
+    const int nr = nb * N, step = 3 * TS;  // the tables of consecutive roots and primitive quartets follow each other
+#pragma unroll 2
+    for (int r = 0; r < nr; ++r) {
+      const double xy = X[r * step] * Y[r * step];
+#pragma unroll
+      for (int k = 0; k < NZ; ++k)
+        if (k < nz) v[k] = fma(xy, Z[r * step + k], v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < NZ; ++k)
+      if (k < nz) acc[(size_t)(ib_cidx(fx, fy, z0 + k) - d.f0) * d.ne + e] += v[k];
+  }
+}
+
+// Adds the [e0|f0] of the n <= IB_GEN_SUB primitive quartets c0 + live[] to acc
+// ([f][e]); the whole block.
+__device__ __forceinline__ void ib_gen_primitives(const IbLaunch& a, int n, int c0,
+                                                  const unsigned short* __restrict__ live, const IbGenShared& sh,
+                                                  const IbGenericDims& d, double RAB2, double RCD2,
+                                                  double* __restrict__ acc, int tab_doubles,
+                                                  const unsigned short* __restrict__ ct,
+                                                  const unsigned char* __restrict__ cp) {
+  extern __shared__ double ib_smem[];
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int N = d.L / 2 + 1, C1 = d.F + 1, TS = ((d.E + 1) * C1) | 1;
+  const int NB = min(IB_GEN_SUB, tab_doubles / (3 * N * TS));
+  double* __restrict__ fld = ib_smem;
+  double* __restrict__ uw = ib_smem + IB_GEN_O_UW;
+  double* __restrict__ tab = ib_smem + IB_GEN_O_TAB;
+  __syncthreads();  // live[] is written, the previous fields and tables are read
+  if (tid < n) {
+    int r = c0 + live[tid];
+    const int id = r % sh.k[3]; r /= sh.k[3];
+    const int ic = r % sh.k[2]; r /= sh.k[2];
+    const int ib = r % sh.k[1]; r /= sh.k[1];
+    const int ia = r;
+    const double xa = a.prim_exp[sh.ptr[0] + ia], ca = a.prim_coef[sh.ptr[0] + ia];
+    const double xb = a.prim_exp[sh.ptr[1] + ib], cb = a.prim_coef[sh.ptr[1] + ib];
+    const double xc = a.prim_exp[sh.ptr[2] + ic], cc = a.prim_coef[sh.ptr[2] + ic];
+    const double xd = a.prim_exp[sh.ptr[3] + id], cd = a.prim_coef[sh.ptr[3] + id];
+    const double zeta = xa + xb, oz = 1.0 / zeta, eta = xc + xd, oe = 1.0 / eta;
+    const double ozpe = 1.0 / (zeta + eta), rho = zeta * eta * ozpe;
+    double r2 = 0.0;
+    double* __restrict__ o = fld + tid * IB_GEN_FLD;
+    for (int c = 0; c < 3; ++c) {
+      const double PA = -xb * oz * sh.AB[c], QC = -xd * oe * sh.CD[c];
+      const double PQ = (sh.A[c] + PA) - (sh.C[c] + QC);
+      r2 = fma(PQ, PQ, r2);
+      o[c] = PA;
+      o[3 + c] = -rho * oz * PQ;  // W - P
+      o[6 + c] = QC;
+      o[9 + c] = rho * oe * PQ;   // W - Q
+    }
+    o[12] = 0.5 * oz;
+    o[13] = rho * oz;
+    o[14] = 0.5 * oe;
+    o[15] = rho * oe;
+    o[16] = 0.5 * ozpe;
+    o[17] = rho * r2;
+    o[18] = ib_two_pi52() * oz * oe * sqrt(ozpe) * ca * cb * cc * cd * exp(-xa * xb * oz * RAB2 - xc * xd * oe * RCD2);
+  }
+  __syncthreads();
+  for (int x = tid; x < n * N; x += nt) {
+    const int u = x / N, rt = x - u * N;
+    ib_rys_root_rt(a.rys_tab, a.boys_tab, N, fld[u * IB_GEN_FLD + 17], fld[u * IB_GEN_FLD + 18], rt, uw + 2 * x);
+  }
+  for (int b0 = 0; b0 < n; b0 += NB) {
+    const int nb = min(NB, n - b0);
+    __syncthreads();  // the roots are there, the last batch's tables are read
+    for (int x = tid; x < nb * 3 * N; x += nt) {
+      const int u = x / (3 * N), y = x - u * 3 * N, rt = y / 3, c = y - 3 * rt;
+      const double* __restrict__ f = fld + (b0 + u) * IB_GEN_FLD;
+      const double t = uw[2 * ((b0 + u) * N + rt)];
+      const double C = fma(t, f[3 + c], f[c]), D = fma(t, f[9 + c], f[6 + c]);
+      const double B10 = f[12] * (1.0 - t * f[13]), B01 = f[14] * (1.0 - t * f[15]), B00 = t * f[16];
+      double* __restrict__ tb = tab + (size_t)x * TS;
+      double p0 = 0.0, p1 = c == 2 ? uw[2 * ((b0 + u) * N + rt) + 1] : 1.0;
+      tb[0] = p1;
+      for (int e = 0; e < d.E; ++e) {
+        const double v = fma(C, p1, e * B10 * p0);
+        tb[(e + 1) * C1] = v;
+        p0 = p1;
+        p1 = v;
+      }
+      for (int fl = 0; fl < d.F; ++fl) {
+        double below = 0.0;  // I(e - 1, fl)
+        for (int e = 0; e <= d.E; ++e) {
+          const double here = tb[e * C1 + fl];
+          double v = fma(D, here, e * B00 * below);
+          if (fl) v = fma(fl * B01, tb[e * C1 + fl - 1], v);
+          tb[e * C1 + fl + 1] = v;
+          below = here;
+        }
+      }
+    }
+    __syncthreads();
+    switch (d.ld) {  // f_z of one (f_x, f_y): l_d + 1 at most
+      case 0: ib_gen_products<1>(nb, N, d, acc, tab, ct, cp); break;
+      case 1: ib_gen_products<2>(nb, N, d, acc, tab, ct, cp); break;
+      case 2: ib_gen_products<3>(nb, N, d, acc, tab, ct, cp); break;
+      case 3: ib_gen_products<4>(nb, N, d, acc, tab, ct, cp); break;
+      case 4: ib_gen_products<5>(nb, N, d, acc, tab, ct, cp); break;
+      default: ib_gen_products<7>(nb, N, d, acc, tab, ct, cp); break;
+    }
+  }
+}
+
 // One contracted quartet, sorted item p, in the block's scratch slice w.
 // CS > 1: this block is rank crank of the CS blocks of a cluster that evaluate
 // the quartet together (every rank calls this with the same p); wc is rank 0's
@@ -139,7 +267,8 @@ __device__ __forceinline__ void ib_gen_item(const IbLaunch& a, int p, int sph, d
                                             double* __restrict__ wc, long long slice, int crank, IbGenShared& sh,
                                             const unsigned short* __restrict__ ct,
                                             const unsigned short* __restrict__ em,
-                                            const unsigned short* __restrict__ eu) {
+                                            const unsigned short* __restrict__ eu,
+                                            const unsigned char* __restrict__ cp, int smem_tab) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int tid = threadIdx.x, nt = blockDim.x;
     if (tid == 0) {
@@ -199,8 +328,6 @@ __device__ __forceinline__ void ib_gen_item(const IbLaunch& a, int p, int sph, d
       break;
     }
     double* acc = w + d.o_acc;
-    double* bra = w + d.o_bra;
-    double* ket = w + d.o_ket;
     for (int i = tid; i < d.ne * d.nf; i += nt) acc[i] = 0.0;
     const double RAB2 = sh.AB[0] * sh.AB[0] + sh.AB[1] * sh.AB[1] + sh.AB[2] * sh.AB[2];
     const double RCD2 = sh.CD[0] * sh.CD[0] + sh.CD[1] * sh.CD[1] + sh.CD[2] * sh.CD[2];
@@ -248,109 +375,8 @@ __device__ __forceinline__ void ib_gen_item(const IbLaunch& a, int p, int sph, d
         __syncthreads();  // sh.wcnt is rewritten by the next round
       }
       const int nmine = ranks_below(base) - mine0;
-    for (int li = 0; li < nmine; ++li) {
-      const int pq = c0 + sh.live[li];
-      __syncthreads();
-      if (tid == 0) {
-        int r = pq;
-        const int id = r % sh.k[3]; r /= sh.k[3];
-        const int ic = r % sh.k[2]; r /= sh.k[2];
-        const int ib = r % sh.k[1]; r /= sh.k[1];
-        const int ia = r;
-        const double xa = a.prim_exp[sh.ptr[0] + ia], ca = a.prim_coef[sh.ptr[0] + ia];
-        const double xb = a.prim_exp[sh.ptr[1] + ib], cb = a.prim_coef[sh.ptr[1] + ib];
-        const double xc = a.prim_exp[sh.ptr[2] + ic], cc = a.prim_coef[sh.ptr[2] + ic];
-        const double xd = a.prim_exp[sh.ptr[3] + id], cd = a.prim_coef[sh.ptr[3] + id];
-        const double zeta = xa + xb, oz = 1.0 / zeta, eta = xc + xd, oe = 1.0 / eta;
-        const double ozpe = 1.0 / (zeta + eta), rho = zeta * eta * ozpe;
-        double P[3], Q[3], PQ[3];
-        for (int c = 0; c < 3; ++c) {
-          P[c] = (xa * sh.A[c] + xb * sh.B[c]) * oz;
-          Q[c] = (xc * sh.C[c] + xd * sh.D[c]) * oe;
-          PQ[c] = P[c] - Q[c];
-          const double W = (zeta * P[c] + eta * Q[c]) * ozpe;
-          sh.PA[c] = P[c] - sh.A[c];
-          sh.WP[c] = W - P[c];
-          sh.QC[c] = Q[c] - sh.C[c];
-          sh.WQ[c] = W - Q[c];
-        }
-        sh.o2z = 0.5 * oz;
-        sh.roz = rho * oz;
-        sh.o2e = 0.5 * oe;
-        sh.roe = rho * oe;
-        sh.o2zpe = 0.5 * ozpe;
-        const double RPQ2 = PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2];
-        ib_boys_rt(rho * RPQ2, d.L, a.boys_tab, sh.F);
-        const double pref = ib_two_pi52() * oz * oe * sqrt(ozpe) * ca * cb * cc * cd *
-                            exp(-xa * xb * oz * RAB2 - xc * xd * oe * RCD2);
-        for (int m = 0; m <= d.L; ++m) sh.F[m] *= pref;
-      }
-      __syncthreads();
-      // ---- bra VRR, level by level: bra[m*ncumE + e]
-      for (int m = tid; m <= d.L; m += nt) {
-        bra[m * d.ncumE] = sh.F[m];
-        if (m == 0 && d.lc == 0 && d.la == 0) acc[0] += sh.F[0];
-      }
-      for (int le = 1; le <= d.E; ++le) {
-        __syncthreads();
-        const int nce = ib_ncart(le), nm = d.L - le + 1;
-        for (int idx = tid; idx < nce * nm; idx += nt) {
-          const int m = idx / nce, e = ib_ncum(le - 1) + idx % nce;
-          int ex, ey, ez;
-          ib_ct_get(ct, e, ex, ey, ez);
-          const int i = ib_gen_dir(ex, ey);
-          const unsigned t1 = em[i * IB_GEN_NCT + e];
-          const int e1 = t1 & 511, n = (int)(t1 >> 9) - 1;  // e - 1_i, its exponent along i
-          double v = sh.PA[i] * bra[m * d.ncumE + e1] + sh.WP[i] * bra[(m + 1) * d.ncumE + e1];
-          if (n > 0) {
-            const int e2 = em[i * IB_GEN_NCT + e1] & 511;  // e - 2_i
-            v += n * sh.o2z * (bra[m * d.ncumE + e2] - sh.roz * bra[(m + 1) * d.ncumE + e2]);
-          }
-          bra[m * d.ncumE + e] = v;
-          if (m == 0 && d.lc == 0 && e >= d.e0) acc[e - d.e0] += v;  // f = 0 column of [f][e]
-        }
-      }
-      // ---- ket VRR: level f stored at ket + koff(f) as [m][fcomp][e].  One warp per
-      // row (m, fcomp): the f-side indices once per row; its lanes run over e, with
-      // e - 1_i and the exponent of e along i from the table em
-      for (int lf = 1; lf <= d.F; ++lf) {
-        __syncthreads();
-        const int ncf = ib_ncart(lf), nm = d.F - lf + 1, E_ = d.ncumE;
-        double* dst = ket + ib_koff(d, lf);
-        const double* s1 = lf == 1 ? bra : ket + ib_koff(d, lf - 1);
-        const double* s2 = lf <= 2 ? bra : ket + ib_koff(d, lf - 2);  // read only when lf >= 2
-        const int nc1 = ib_ncart(lf - 1), nc2 = ib_ncart(lf - 2);
-        for (int row = warp; row < nm * ncf; row += nwarp) {
-          const int m = row / ncf, fc = row - m * ncf;
-          int fx, fy, fz;
-          ib_ct_get(ct, ib_ncum(lf - 1) + fc, fx, fy, fz);
-          const int i = ib_gen_dir(fx, fy);
-          const unsigned tf = em[i * IB_GEN_NCT + ib_ncum(lf - 1) + fc];
-          const int nn = (int)(tf >> 9) - 1;              // exponent of f - 1_i along i
-          const int f1 = (int)(tf & 511) - ib_ncum(lf - 2);  // in-level index of f - 1_i at lf-1
-          int f2 = 0;
-          if (nn > 0) f2 = (int)(em[i * IB_GEN_NCT + (tf & 511)] & 511) - ib_ncum(lf - 3);  // f - 2_i
-          const double qc = sh.QC[i], wq = sh.WQ[i], t2 = nn * sh.o2e, roe = sh.roe, o2zpe = sh.o2zpe;
-          const double* __restrict__ r10 = s1 + ((size_t)m * nc1 + f1) * E_;
-          const double* __restrict__ r11 = s1 + ((size_t)(m + 1) * nc1 + f1) * E_;
-          const double* __restrict__ r20 = s2 + ((size_t)m * nc2 + f2) * E_;
-          const double* __restrict__ r21 = s2 + ((size_t)(m + 1) * nc2 + f2) * E_;
-          double* __restrict__ out = dst + ((size_t)m * ncf + fc) * E_;
-          const unsigned short* emi = em + i * IB_GEN_NCT;
-          const bool to_acc = m == 0 && lf >= d.lc;
-          double* accc = acc + (size_t)(ib_ncum(lf - 1) + fc - d.f0) * d.ne;  // this f's row of [f][e]
-#pragma unroll 4
-          for (int e = lane; e < E_; e += 32) {  // unrolled: the lanes' loads of several e issue together
-            double v = qc * r10[e] + wq * r11[e];
-            if (nn > 0) v += t2 * (r20[e] - roe * r21[e]);
-            const unsigned t = emi[e];
-            if (t >> 9) v += (double)(t >> 9) * o2zpe * r11[t & 511];
-            out[e] = v;
-            if (to_acc && e >= d.e0) accc[e - d.e0] += v;
-          }
-        }
-      }
-    }  // this rank's live primitive quartets of the chunk
+      for (int s0 = 0; s0 < nmine; s0 += IB_GEN_SUB)
+        ib_gen_primitives(a, min(IB_GEN_SUB, nmine - s0), c0, sh.live + s0, sh, d, RAB2, RCD2, acc, smem_tab, ct, cp);
     }  // chunk
     __syncthreads();
     if (CS > 1) {
@@ -472,13 +498,17 @@ __device__ __forceinline__ void ib_gen_item(const IbLaunch& a, int p, int sph, d
 // items are shared by a cluster, the light ones taken by single blocks.
 template <int MINB, int CS>
 __global__ void __launch_bounds__(IB_GEN_BLOCK, MINB) ib_eri_generic(const IbLaunch a, const IbGenWork wk, int sph,
-                                                                     double* __restrict__ scratch, long long slice) {
+                                                                     double* __restrict__ scratch, long long slice, int smem_tab) {
   __shared__ IbGenShared sh;
   __shared__ unsigned short ct[IB_GEN_NCT];
   __shared__ unsigned short em[3 * IB_GEN_NCT];
   __shared__ unsigned short eu[3 * IB_GEN_NCT];
+  __shared__ unsigned char cp[(2 * IB_LMAX + 1) * (IB_LMAX + 1)];  // (f_x, f_y) pairs by f_x + f_y
   __shared__ int ticket;
   ib_gen_tables(ct, em, eu);
+  if (threadIdx.x <= 2 * IB_LMAX)
+    for (int y = 0; y <= (int)threadIdx.x; ++y)
+      cp[threadIdx.x * (threadIdx.x + 1) / 2 + y] = (unsigned char)((threadIdx.x - y) | (y << 4));
   __syncthreads();
   const int tid = threadIdx.x;
   int crank = 0;
@@ -504,7 +534,7 @@ __global__ void __launch_bounds__(IB_GEN_BLOCK, MINB) ib_eri_generic(const IbLau
     return wk.redo ? a.redo[2 + a.redo_cap - 1 - t] : lb + t;
   };
   if (!wk.tickets) {  // fixed order, one block per item
-    for (int t = blockIdx.x; t < nh + nl; t += gridDim.x) ib_gen_item<1>(a, item(t), sph, w, w, slice, 0, sh, ct, em, eu);
+    for (int t = blockIdx.x; t < nh + nl; t += gridDim.x) ib_gen_item<1>(a, item(t), sph, w, w, slice, 0, sh, ct, em, eu, cp, smem_tab);
     return;
   }
   if constexpr (CS > 1) {
@@ -515,7 +545,7 @@ __global__ void __launch_bounds__(IB_GEN_BLOCK, MINB) ib_eri_generic(const IbLau
       const int t = *cl.map_shared_rank(&ticket, 0);
       cl.sync();  // read by every rank before rank 0 takes the next ticket
       if (t >= nh) break;
-      ib_gen_item<CS>(a, item(t), sph, w, wc, slice, crank, sh, ct, em, eu);
+      ib_gen_item<CS>(a, item(t), sph, w, wc, slice, crank, sh, ct, em, eu, cp, smem_tab);
     }
   } else {
     for (;;) {
@@ -524,7 +554,7 @@ __global__ void __launch_bounds__(IB_GEN_BLOCK, MINB) ib_eri_generic(const IbLau
       const int t = ticket;
       __syncthreads();
       if (t >= nh) break;
-      ib_gen_item<1>(a, item(t), sph, w, w, slice, 0, sh, ct, em, eu);
+      ib_gen_item<1>(a, item(t), sph, w, w, slice, 0, sh, ct, em, eu, cp, smem_tab);
     }
   }
   for (;;) {
@@ -533,7 +563,7 @@ __global__ void __launch_bounds__(IB_GEN_BLOCK, MINB) ib_eri_generic(const IbLau
     const int t = ticket;
     __syncthreads();
     if (t >= nl) break;
-    ib_gen_item<1>(a, item(nh + t), sph, w, w, slice, 0, sh, ct, em, eu);
+    ib_gen_item<1>(a, item(nh + t), sph, w, w, slice, 0, sh, ct, em, eu, cp, smem_tab);
   }
 }
 
@@ -570,6 +600,24 @@ int ib_generic_split_min() {
 
 namespace {
 
+// Dynamic shared memory of a block: with 2 blocks per SM 100 KB (five (gg|gg)
+// primitive quartets' tables at once); with more the 66 KB that one primitive
+// quartet of l = 6 needs (three blocks then fit an SM).
+template <int MINB>
+constexpr int gen_smem() {
+  return (MINB <= 2 ? 100 : 66) * 1024;
+}
+template <int MINB>
+constexpr int gen_tab() {
+  return gen_smem<MINB>() / 8 - IB_GEN_O_TAB;
+}
+static_assert(gen_tab<4>() >= 3 * 13 * 13 * 13, "tables of one primitive quartet with l = 6 on all shells");
+
+template <int MINB, int CS>
+cudaError_t gen_prepare() {  // on every launch: the attribute is per device, and setting it costs little
+  return cudaFuncSetAttribute(ib_eri_generic<MINB, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, gen_smem<MINB>());
+}
+
 // Clusters of CS blocks of the split kernel resident at once on the current
 // device (cached per device; 0 when the device cannot hold one).
 template <int MINB, int CS>
@@ -587,9 +635,14 @@ int split_clusters_resident() {
   at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(CS);
   cfg.blockDim = dim3(IB_GEN_BLOCK);
+  cfg.dynamicSmemBytes = gen_smem<MINB>();
   cfg.attrs = at;
   cfg.numAttrs = 1;
   int n = 0;
+  if (gen_prepare<MINB, CS>() != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
   if (cudaOccupancyMaxActiveClusters(&n, ib_eri_generic<MINB, CS>, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;  // this launch without clusters; asked again next time
@@ -613,12 +666,15 @@ cudaError_t launch_split(int grid, cudaStream_t s, const IbLaunch& a, const IbGe
     at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(clusters * CS);
     cfg.blockDim = dim3(IB_GEN_BLOCK);
+    cfg.dynamicSmemBytes = gen_smem<MINB>();
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, ib_eri_generic<MINB, CS>, a, wk, sph, scratch, slice);
+    return cudaLaunchKernelEx(&cfg, ib_eri_generic<MINB, CS>, a, wk, sph, scratch, slice, gen_tab<MINB>());
   }
-  ib_eri_generic<MINB, 1><<<grid, IB_GEN_BLOCK, 0, s>>>(a, wk, sph, scratch, slice);
+  const cudaError_t e = gen_prepare<MINB, 1>();
+  if (e != cudaSuccess) return e;
+  ib_eri_generic<MINB, 1><<<grid, IB_GEN_BLOCK, gen_smem<MINB>(), s>>>(a, wk, sph, scratch, slice, gen_tab<MINB>());
   return cudaGetLastError();
 }
 
@@ -627,7 +683,9 @@ cudaError_t launch_bps(int grid, cudaStream_t s, const IbLaunch& a, const IbGenW
                        long long slice) {
   if (wk.tickets && wk.split >= 4) return launch_split<MINB, 4>(grid, s, a, wk, sph, scratch, slice);
   if (wk.tickets && wk.split >= 2) return launch_split<MINB, 2>(grid, s, a, wk, sph, scratch, slice);
-  ib_eri_generic<MINB, 1><<<grid, IB_GEN_BLOCK, 0, s>>>(a, wk, sph, scratch, slice);
+  const cudaError_t e = gen_prepare<MINB, 1>();
+  if (e != cudaSuccess) return e;
+  ib_eri_generic<MINB, 1><<<grid, IB_GEN_BLOCK, gen_smem<MINB>(), s>>>(a, wk, sph, scratch, slice, gen_tab<MINB>());
   return cudaGetLastError();
 }
 

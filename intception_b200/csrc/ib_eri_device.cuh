@@ -942,13 +942,11 @@ __device__ __forceinline__ void ib_boys_row(double T, const double* __restrict__
   }
 }
 
-// Root rt of N at Boys argument T: (u, weight x pref).
-template <int N>
-__device__ __forceinline__ void ib_rys_root(const double* __restrict__ tab, double T, double pref, int rt,
+// Root rt of N >= 2 at Boys argument T: (u, weight x pref).
+__device__ __forceinline__ void ib_rys_eval(const double2* __restrict__ t, int N, int tmax, double T, double pref,
                                             double* __restrict__ dst) {
-  const double2* __restrict__ t = reinterpret_cast<const double2*>(tab + ib_rys_off(N)) + rt;
   double2 v;
-  if (T < (double)ib_rys_tmax(N)) {
+  if (T < (double)tmax) {
     const double s = T * (double)IB_RYS_H_INV;
     const int row = (int)s;
     const double x = fma(2.0, s - (double)row, -1.0);
@@ -961,12 +959,29 @@ __device__ __forceinline__ void ib_rys_root(const double* __restrict__ tab, doub
       v.y = fma(v.y, x, c.y);
     }
   } else {
-    const double2 c = __ldg(t + ib_rys_tmax(N) * IB_RYS_H_INV * (IB_RYS_DEG + 1) * N);
+    const double2 c = __ldg(t + tmax * IB_RYS_H_INV * (IB_RYS_DEG + 1) * N);
     const double r = rsqrt(T);
     v.x = c.x * r * r;
     v.y = c.y * r;
   }
   reinterpret_cast<double2*>(dst)[0] = make_double2(v.x, v.y * pref);
+}
+template <int N>
+__device__ __forceinline__ void ib_rys_root(const double* __restrict__ tab, double T, double pref, int rt,
+                                            double* __restrict__ dst) {
+  ib_rys_eval(reinterpret_cast<const double2*>(tab + ib_rys_off(N)) + rt, N, ib_rys_tmax(N), T, pref, dst);
+}
+// N known at run time (the generic kernel), N = 1 included: u = F_1/F_0, weight F_0.
+__device__ inline void ib_rys_root_rt(const double* __restrict__ tab, const double* __restrict__ boys_tab, int N,
+                                      double T, double pref, int rt, double* __restrict__ dst) {
+  if (N == 1) {
+    double F[2];
+    ib_boys_rt(T, 1, boys_tab, F);
+    dst[0] = F[1] / F[0];
+    dst[1] = F[0] * pref;
+    return;
+  }
+  ib_rys_eval(reinterpret_cast<const double2*>(tab + ib_rys_off(N)) + rt, N, ib_rys_tmax(N), T, pref, dst);
 }
 
 template <typename R>

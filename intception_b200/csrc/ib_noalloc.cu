@@ -42,6 +42,7 @@ static __device__ __align__(256) IbItem ib_noalloc_items[IB_NOALLOC_MAX_QUARTETS
 static __device__ __align__(256) int ib_noalloc_ranges[kNoallocRanges];
 static __device__ __align__(256) int ib_noalloc_status;
 static __device__ __align__(256) double ib_noalloc_boys[IB_BOYS_NPTS * IB_BOYS_NCOL];
+static __device__ __align__(256) double ib_noalloc_rys[IB_RYS_SIZE];
 static __device__ __align__(256) double ib_noalloc_sph[kSphDoubles];
 
 struct NoallocDevice {
@@ -52,6 +53,7 @@ struct NoallocDevice {
   int* ranges = nullptr;
   int* status = nullptr;
   double* boys = nullptr;
+  double* rys = nullptr;
   double* sph = nullptr;
 };
 NoallocDevice g_dev[64];
@@ -70,6 +72,9 @@ int noalloc_setup(int dev, NoallocDevice** out) {
     if (cudaGetSymbolAddress((void**)&d.ranges, ib_noalloc_ranges) != cudaSuccess) return IB_ERR_CUDA;
     if (cudaGetSymbolAddress((void**)&d.status, ib_noalloc_status) != cudaSuccess) return IB_ERR_CUDA;
     if (cudaGetSymbolAddress((void**)&d.boys, ib_noalloc_boys) != cudaSuccess) return IB_ERR_CUDA;
+    if (cudaGetSymbolAddress((void**)&d.rys, ib_noalloc_rys) != cudaSuccess) return IB_ERR_CUDA;
+    if (cudaMemcpyToSymbol(ib_noalloc_rys, ib_rys_host_table, sizeof(ib_rys_host_table)) != cudaSuccess)
+      return IB_ERR_CUDA;
     if (cudaGetSymbolAddress((void**)&d.sph, ib_noalloc_sph) != cudaSuccess) return IB_ERR_CUDA;
     if (cudaMemcpyToSymbol(ib_noalloc_boys, ib_boys_host_table, sizeof(ib_boys_host_table)) != cudaSuccess)
       return IB_ERR_CUDA;
@@ -203,6 +208,7 @@ extern "C" int intception_b200_eri_batch_noalloc(const intception_b200_basis* ba
   a.prim_exp = basis->prim_exp;
   a.prim_coef = basis->prim_coef;
   a.boys_tab = d->boys;
+  a.rys_tab = d->rys;
   a.sph = d->sph;
   a.out = out;
   a.status = d->status;

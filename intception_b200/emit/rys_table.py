@@ -10,8 +10,7 @@ polynomial and the Christoffel numbers, all in 60-digit arithmetic.
 
 Between 0 and RYS_TMAX[N] each root and weight is a polynomial of degree
 RYS_DEG in x = 2 (4 T - row) - 1 on the interval [row/4, (row + 1)/4)
-(interpolation at the Chebyshev nodes: at most 6e-17 relative error for
-N <= 9).  Above RYS_TMAX[N] the rule is the half-range Hermite one,
+(interpolation at the Chebyshev nodes: at most 6e-17 relative error).  Above RYS_TMAX[N] the rule is the half-range Hermite one,
 u_r = h_r / T, w_r = v_r / sqrt(T), within 1e-16 relative.
 
 Layout per N, in doubles: rows x (RYS_DEG + 1) x N x (root, weight), then
@@ -24,8 +23,8 @@ import sys
 
 RYS_H_INV = 4            # intervals per unit T
 RYS_DEG = 8
-RYS_NMIN, RYS_NMAX = 2, 9
-RYS_TMAX = {2: 47, 3: 54, 4: 60, 5: 66, 6: 72, 7: 78, 8: 84, 9: 90}
+RYS_NMIN, RYS_NMAX = 2, 13   # 13: l = 6 on all four shells
+RYS_TMAX = {2: 47, 3: 54, 4: 60, 5: 66, 6: 72, 7: 78, 8: 84, 9: 90, 10: 95, 11: 100, 12: 105, 13: 110}
 
 
 def _moments(T, n):
@@ -118,7 +117,7 @@ def _asymptotic(N):
 
 def write_headers(outdir):
     """rys_table.h (sizes) and rys_table_data.h (the values).  The values take
-    about two minutes of one core; they are kept while this file is unchanged."""
+    about five minutes of one core; they are kept while this file is unchanged."""
     from .boys_table import _write
     import hashlib
     with open(os.path.abspath(__file__), 'rb') as fh:
@@ -136,6 +135,7 @@ def write_headers(outdir):
         '#define IB_RYS_DEG %d' % RYS_DEG,
         '#define IB_RYS_NMAX %d' % RYS_NMAX,
         '#define IB_RYS_SIZE %d' % off,
+        'extern const double ib_rys_host_table[IB_RYS_SIZE];',
         '__host__ __device__ inline constexpr int ib_rys_off(int N) { return %s; }' % pick(offs),
         '__host__ __device__ inline constexpr int ib_rys_tmax(int N) { return %s; }' % pick(RYS_TMAX)])
     if os.path.exists(data):
@@ -153,7 +153,7 @@ def write_headers(outdir):
             raise RuntimeError('rys_table: a worker failed')
         got.update((int(row), {int(N): c for N, c in cs.items()}) for row, cs in json.loads(text).items())
     lines = ['/* %s: generated by intception_b200/emit/rys_table.py. */' % key, '#pragma once', '#include "rys_table.h"',
-             'static const double ib_rys_host_table[IB_RYS_SIZE] = {']
+             'const double ib_rys_host_table[IB_RYS_SIZE] = {']
     for N in range(RYS_NMIN, RYS_NMAX + 1):
         for row in range(RYS_TMAX[N] * RYS_H_INV):
             c = got[row][N]
