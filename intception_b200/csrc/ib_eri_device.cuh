@@ -13,6 +13,10 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <cmath>
+#include <vector>
+
 #include "_gen/boys_table.h"
 #include "_gen/rys_table.h"
 
@@ -895,6 +899,21 @@ __device__ __forceinline__ void ib_rys_setup(const double* __restrict__ pab, con
   o[9 * 32] = q.T;
   o[10 * 32] = q.pref;
   o[11 * 32] = q.fd;
+}
+
+// Rows of ib_boys_row for L = 0..lmax from the full table (rows of IB_BOYS_NCOL values F_n(T_i)).
+inline void ib_boys_rows_host(const double* table, int lmax, std::vector<double>& rows) {
+  rows.assign((size_t)(lmax + 1) * IB_BOYS_NPTS * 8, 0.0);
+  for (int L = 0; L <= lmax; ++L)
+    for (int i = 0; i < IB_BOYS_NPTS; ++i) {
+      double* row = rows.data() + ((size_t)L * IB_BOYS_NPTS + i) * 8;
+      double fact = 1.0;
+      for (int k = 0; k < IB_BOYS_TAYLOR; ++k) {
+        row[k] = table[i * IB_BOYS_NCOL + L + k] / fact;
+        fact *= k + 1;
+      }
+      row[7] = std::exp(-(double)i / IB_BOYS_H_INV);
+    }
 }
 
 // F_0..F_L(T) for the lane-per-primitive kernels.  Row i of L holds F_(L+k)(T_i)/k!,

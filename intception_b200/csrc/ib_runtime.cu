@@ -559,17 +559,8 @@ int get_context(Context** out) {
     IB_CUDA(cudaMemcpy(c->boys_tab.p, ib_boys_host_table, sizeof(ib_boys_host_table), cudaMemcpyHostToDevice));
     IB_CUDA(c->rys_tab.ensure(sizeof(ib_rys_host_table)));
     IB_CUDA(cudaMemcpy(c->rys_tab.p, ib_rys_host_table, sizeof(ib_rys_host_table), cudaMemcpyHostToDevice));
-    std::vector<double> rows((size_t)(IB_BOYS_ROW_LMAX + 1) * IB_BOYS_NPTS * 8);
-    for (int L = 0; L <= IB_BOYS_ROW_LMAX; ++L)
-      for (int i = 0; i < IB_BOYS_NPTS; ++i) {
-        double* row = rows.data() + ((size_t)L * IB_BOYS_NPTS + i) * 8;
-        double fact = 1.0;
-        for (int k = 0; k < IB_BOYS_TAYLOR; ++k) {
-          row[k] = ib_boys_host_table[i * IB_BOYS_NCOL + L + k] / fact;
-          fact *= k + 1;
-        }
-        row[7] = std::exp(-(double)i / IB_BOYS_H_INV);
-      }
+    std::vector<double> rows;
+    ib_boys_rows_host(ib_boys_host_table, IB_BOYS_ROW_LMAX, rows);
     IB_CUDA(c->boys_row.ensure(rows.size() * sizeof(double)));
     IB_CUDA(cudaMemcpy(c->boys_row.p, rows.data(), rows.size() * sizeof(double), cudaMemcpyHostToDevice));
     std::vector<double> sph;

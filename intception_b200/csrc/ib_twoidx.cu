@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <vector>
 
 #include "../../include/intception_b200.h"
 #include "_gen/boys_table_data.h"
@@ -43,6 +44,7 @@ int ib_runtime_set_status(int st, const char* msg);
 namespace {
 
 static __device__ __align__(256) double ib2_boys[IB_BOYS_NPTS * IB_BOYS_NCOL];
+static __device__ __align__(256) double ib2_rows[5 * IB_BOYS_NPTS * 8];  // ib_boys_row's rows, L = 0..4
 
 struct Ib2Args {
   int n;
@@ -57,6 +59,7 @@ struct Ib2Args {
   const long long* off;
   double* out;
   const double* boys;
+  const double* rows;
   int* status;
   int lthr;  // lane-group kernels: pairs with max(la, lb) <= lthr belong to the thread-per-pair kernels
   int bulk_ok;  // thread-per-pair kernel: every input array 16-byte aligned (complete chunks by bulk copy)
@@ -289,41 +292,11 @@ __host__ __device__ constexpr int ib2_hrr_max(int LA, int LB) {
   return h;
 }
 
-// F_m(T), m = 0..L, reading the global table (no staging; L is a constant).
-template <int L>
-__device__ __forceinline__ void ib2_boys_f(double T, const double* __restrict__ tab, double* F) {
-  if (T < IB_BOYS_TMAX) {
-    const int i = __double2int_rn(T * (double)IB_BOYS_H_INV);
-    const double dx = (double)i * (1.0 / IB_BOYS_H_INV) - T;
-    const double* r = tab + i * IB_BOYS_NCOL + L;
-    double f = __ldg(r + 6) * (1.0 / 720.0);
-    f = fma(f, dx, __ldg(r + 5) * (1.0 / 120.0));
-    f = fma(f, dx, __ldg(r + 4) * (1.0 / 24.0));
-    f = fma(f, dx, __ldg(r + 3) * (1.0 / 6.0));
-    f = fma(f, dx, __ldg(r + 2) * 0.5);
-    f = fma(f, dx, __ldg(r + 1));
-    F[L] = fma(f, dx, __ldg(r));
-    if (L > 0) {
-      const double e = exp(-T), t2 = T + T;
-#pragma unroll
-      for (int m = L - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], e) * (1.0 / (2 * m + 1));
-    }
-  } else {
-    const double oT = 1.0 / T;
-    F[0] = sqrt(0.78539816339744830962 * oT);  // (1/2) sqrt(pi/T)
-    if (L > 0) {
-      const double he = 0.5 * exp(-T);
-#pragma unroll
-      for (int m = 0; m < L; ++m) F[m + 1] = fma((double)m + 0.5, F[m], -he) * oT;
-    }
-  }
-}
-
 // Nuclear attraction of one pair, LA >= LB; element (k of LA, f of LB) to o[k*sa + f*sb].
 template <int LA, int LB>
 __device__ __forceinline__ void ib2_nuclear_pair(double xa, const double* __restrict__ pa, double xb,
                                                  const double* __restrict__ pb, const double* __restrict__ pc,
-                                                 const double* __restrict__ boys, double* __restrict__ o, int sa,
+                                                 const double* __restrict__ rows, double* __restrict__ o, int sa,
                                                  int sb) {
   constexpr int L = LA + LB;
   const double op = 1.0 / (xa + xb), o2p = 0.5 * op, xi = xa * xb * op;
@@ -338,7 +311,7 @@ __device__ __forceinline__ void ib2_nuclear_pair(double xa, const double* __rest
     pc2 = fma(PC[d], PC[d], pc2);
   }
   double V[ib2_vrr_off(L + 1, L)];
-  ib2_boys_f<L>((xa + xb) * pc2, boys, V);
+  ib_boys_row<L>((xa + xb) * pc2, rows, V);
   const double pref = 6.283185307179586477 * op * exp(-xi * ab2);
 #pragma unroll
   for (int m = 0; m <= L; ++m) V[m] *= pref;
@@ -454,18 +427,28 @@ __device__ __forceinline__ void ib2_overlap_pair(double xa, const double* __rest
 }
 
 // Block-cooperative chunks: a block stages IB2_CHUNK pairs' inputs in shared
-// memory (coalesced, each input byte read once), counting-sorts them by class
-// there, and its warps run the sorted list, so the 32 lanes of a warp execute
-// the same unrolled class code.  Pairs of the lane-group kernel and refused
-// pairs are left out of the list.
+// memory (coalesced, each input byte read once), sorts them by class there
+// (ballots; no atomics), and its warps run the sorted list, so that nearly all
+// lanes of a warp execute the same unrolled class code.  Pairs of the
+// lane-group kernel and refused pairs are left out of the list.
+//
+// When the chunk's blocks are one contiguous run of the output (packed
+// offsets, every pair evaluated here), the lanes write them to shared memory
+// and the block copies the run out coalesced; a lane's own element stores go
+// to 32 sectors a warp.  Other chunks store directly.
 //
 // The inputs of a complete chunk are contiguous byte ranges of the caller's
-// arrays; they are fetched by bulk copies (TMA, cp.async.bulk) into one of two
-// chunk buffers while the block evaluates the other, with completion counted
-// on an mbarrier per buffer.  The last (partial) chunk, and callers whose
-// arrays are not 16-byte aligned, take plain loads.
+// arrays; they are fetched by bulk copies (TMA, cp.async.bulk) with completion
+// counted on an mbarrier, issued as soon as the previous chunk is evaluated:
+// they arrive while its results are copied out and while the other block of
+// the SM evaluates.  The last (partial) chunk, and callers whose arrays are
+// not 16-byte aligned, take plain loads.
+//
+// 4e6 pairs, l <= 2, one B200: see the figures at ib2_thread_kernel.
 #define IB2_CHUNK 512
 #define IB2_TPB 256
+#define IB2_WR (IB2_CHUNK / 32)  // warp rounds of a chunk
+#define IB2_OUT 6656             // staged output doubles: packed l <= 2 chunks average 5 690, sigma 250
 
 // One chunk's inputs; every member is a whole number of 16-byte units.
 template <int KIND>
@@ -479,12 +462,14 @@ struct Ib2Buf {
 
 template <int KIND>
 struct Ib2Stage {
-  Ib2Buf<KIND> buf[2];
-  unsigned long long full[2];  // mbarrier of each buffer: complete when its bulk copies have landed
+  Ib2Buf<KIND> buf;
+  double out[IB2_OUT];
+  unsigned long long full;    // mbarrier: complete when a chunk's bulk copies have landed
   short order[IB2_CHUNK];     // chunk-local pair index, sorted by class
   unsigned char cls[IB2_CHUNK];
   unsigned char swp[IB2_CHUNK];
-  int count[16], start[16];
+  int cnt[IB2_WR][16];        // per warp round: pairs of each class, then their first position in it
+  int start[17];
 };
 
 __device__ __forceinline__ unsigned ib2_smem_addr(const void* p) {
@@ -539,11 +524,10 @@ __device__ __forceinline__ bool ib2_wait(unsigned mb, unsigned parity, int iters
 
 template <int KIND>
 __device__ __forceinline__ void ib2_thread_pair(const Ib2Buf<KIND>& st, const unsigned char* swp, int c, int j,
-                                                const double* boys, double* out) {
+                                                const double* rows, double* __restrict__ o) {
   if (KIND == 0) {
     const double* pa = st.ca + 3 * j;
     const double* pb = st.cb + 3 * j;
-    double* o = out + st.off[j];
     const double xa = st.xa[j], xb = st.xb[j];
     switch (c) {
       case 0: ib2_overlap_pair<0, 0>(xa, pa, xb, pb, o); break;
@@ -561,10 +545,9 @@ __device__ __forceinline__ void ib2_thread_pair(const Ib2Buf<KIND>& st, const un
     const double* pa = swap ? st.cb + 3 * j : st.ca + 3 * j;
     const double* pb = swap ? st.ca + 3 * j : st.cb + 3 * j;
     const double xa = swap ? st.xb[j] : st.xa[j], xb = swap ? st.xa[j] : st.xb[j];
-    double* o = out + st.off[j];
     const double* pc = st.cc + 3 * j;
 #define IB2_NU(A_, B_)                                                                                      \
-  ib2_nuclear_pair<A_, B_>(xa, pa, xb, pb, pc, boys, o, swap ? ib2_ncart_c(B_) : 1, swap ? 1 : ib2_ncart_c(A_)); \
+  ib2_nuclear_pair<A_, B_>(xa, pa, xb, pb, pc, rows, o, swap ? ib2_ncart_c(B_) : 1, swap ? 1 : ib2_ncart_c(A_)); \
   break;
     switch (c) {
       case 0: IB2_NU(0, 0)
@@ -581,36 +564,31 @@ __device__ __forceinline__ void ib2_thread_pair(const Ib2Buf<KIND>& st, const un
 template <int KIND>
 __global__ void __launch_bounds__(IB2_TPB, 2) ib2_thread_kernel(const Ib2Args a) {
   constexpr int kClasses = KIND == 0 ? (IB2_LT + 1) * (IB2_LT + 1) : (IB2_LT + 1) * (IB2_LT + 2) / 2;
+  constexpr int kRounds = IB2_CHUNK / IB2_TPB;
   extern __shared__ __align__(16) unsigned char ib2_raw[];
   Ib2Stage<KIND>& st = *reinterpret_cast<Ib2Stage<KIND>*>(ib2_raw);
+  Ib2Buf<KIND>& bf = st.buf;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long nchunk = ((long long)a.n + IB2_CHUNK - 1) / IB2_CHUNK;
   const long long nfull = a.bulk_ok ? (long long)a.n / IB2_CHUNK : 0;  // chunks fetched by bulk copies
-  const unsigned mb0 = ib2_smem_addr(&st.full[0]), mb1 = ib2_smem_addr(&st.full[1]);
+  const unsigned mb = ib2_smem_addr(&st.full);
   if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb0) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb1) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if ((long long)blockIdx.x < nfull) ib2_issue<KIND>(a, st.buf[0], blockIdx.x, mb0);
+    if ((long long)blockIdx.x < nfull) ib2_issue<KIND>(a, bf, blockIdx.x, mb);
   }
   __syncthreads();
   int k = 0;
   for (long long ch = blockIdx.x; ch < nchunk; ch += gridDim.x, ++k) {
-    const int b = k & 1;
-    Ib2Buf<KIND>& bf = st.buf[b];
-    const unsigned mb_this = b ? mb1 : mb0, mb_next = b ? mb0 : mb1;
     const long long nxt = ch + gridDim.x;
-    // prefetch the next chunk into the other buffer (read by the previous
-    // iteration, which ended with a block barrier)
-    if (threadIdx.x == 0 && nxt < nfull) ib2_issue<KIND>(a, st.buf[b ^ 1], nxt, mb_next);
     const int p0 = (int)(ch * IB2_CHUNK);
     const int np = min(IB2_CHUNK, a.n - p0);
     if (ch < nfull) {
-      const bool ok = ib2_wait(mb_this, (k >> 1) & 1, a.wait_iters);
-      if (__syncthreads_or(!ok)) {  // uniform: report, drain the copies still in flight, stop
+      const bool ok = ib2_wait(mb, k & 1, a.wait_iters);
+      if (__syncthreads_or(!ok)) {  // uniform: report, drain this chunk's copies (the only ones in flight), stop
         if (threadIdx.x == 0) {
           if (a.status) atomicExch(a.status, IB_ERR_TIMEOUT);
-          ib2_wait(mb_this, (k >> 1) & 1, a.wait_iters);
-          if (nxt < nfull) ib2_wait(mb_next, ((k + 1) >> 1) & 1, a.wait_iters);
+          ib2_wait(mb, k & 1, a.wait_iters);
         }
         return;
       }
@@ -627,47 +605,81 @@ __global__ void __launch_bounds__(IB2_TPB, 2) ib2_thread_kernel(const Ib2Args a)
         bf.cb[t] = __ldg(a.cb + 3LL * p0 + t);
         if (KIND == 1) bf.cc[t] = __ldg(a.cc + 3LL * p0 + t);
       }
+      __syncthreads();
     }
-    if (threadIdx.x < 16) st.count[threadIdx.x] = 0;
-    __syncthreads();
-    // class of every staged pair; per-class counts
-    for (int t = threadIdx.x; t < np; t += IB2_TPB) {
-      const int la = bf.la[t], lb = bf.lb[t];
+    // class of every staged pair, its rank among its class in its warp round,
+    // and whether the chunk's blocks form one run of the output
+    int cl[kRounds], rk[kRounds];
+    bool run = true;
+#pragma unroll
+    for (int q = 0; q < kRounds; ++q) {
+      const int t = threadIdx.x + q * IB2_TPB, wr = q * (IB2_TPB / 32) + warp;
       int c = 255;
-      if (ib2_bad(la, lb, a.lmax, bf.xa[t], bf.xb[t])) {
-        if (a.status) atomicExch(a.status, IB_ERR_ARG);
-      } else if (KIND == 0) {
-        if (la <= IB2_LT && lb <= IB2_LT) c = la * (IB2_LT + 1) + lb;
-      } else {
-        const int hi = max(la, lb), lo = min(la, lb);
-        if (hi <= IB2_LT) c = hi * (hi + 1) / 2 + lo;
-        st.swp[t] = la < lb;
+      if (t < np) {
+        const int la = bf.la[t], lb = bf.lb[t];
+        if (ib2_bad(la, lb, a.lmax, bf.xa[t], bf.xb[t])) {
+          if (a.status) atomicExch(a.status, IB_ERR_ARG);
+        } else if (KIND == 0) {
+          if (la <= IB2_LT && lb <= IB2_LT) c = la * (IB2_LT + 1) + lb;
+        } else {
+          const int hi = max(la, lb), lo = min(la, lb);
+          if (hi <= IB2_LT) c = hi * (hi + 1) / 2 + lo;
+          st.swp[t] = la < lb;
+        }
+        st.cls[t] = (unsigned char)c;
+        const long long end = bf.off[t] + (c == 255 ? 0 : ib2_ncart(la) * ib2_ncart(lb));
+        run = run && c != 255 && (t + 1 < np ? bf.off[t + 1] == end : end - bf.off[0] <= IB2_OUT);
       }
-      st.cls[t] = (unsigned char)c;
-      if (c != 255) atomicAdd(&st.count[c], 1);
+      cl[q] = c;
+      rk[q] = 0;
+#pragma unroll
+      for (int v = 0; v < kClasses; ++v) {
+        const unsigned bal = __ballot_sync(0xffffffffu, c == v);
+        if (c == v) rk[q] = __popc(bal & ((1u << lane) - 1u));
+        if (lane == v) st.cnt[wr][v] = __popc(bal);
+      }
+    }
+    const bool staged = __syncthreads_and(run);
+    if (warp == 0) {
+      int n = 0;
+      if (lane < kClasses)
+        for (int w = 0; w < IB2_WR; ++w) {
+          const int v = st.cnt[w][lane];
+          st.cnt[w][lane] = n;
+          n += v;
+        }
+      int s = n;
+      for (int o = 1; o < 16; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += v;
+      }
+      if (lane < 16) st.start[lane + 1] = s;
+      if (lane == 0) st.start[0] = 0;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int acc = 0;
-      for (int c = 0; c < kClasses; ++c) {
-        st.start[c] = acc;
-        acc += st.count[c];
-      }
-      st.start[kClasses] = acc;
-      for (int c = 0; c < kClasses; ++c) st.count[c] = st.start[c];  // running insert positions
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < np; t += IB2_TPB) {
-      const int c = st.cls[t];
-      if (c != 255) st.order[atomicAdd(&st.count[c], 1)] = (short)t;
-    }
+#pragma unroll
+    for (int q = 0; q < kRounds; ++q)
+      if (cl[q] != 255)
+        st.order[st.start[cl[q]] + st.cnt[q * (IB2_TPB / 32) + warp][cl[q]] + rk[q]] = (short)(threadIdx.x + q * IB2_TPB);
     __syncthreads();
     const int total = st.start[kClasses];
-    for (int i = threadIdx.x; i < total; i += IB2_TPB) {
-      const int j = st.order[i];
-      ib2_thread_pair<KIND>(bf, st.swp, st.cls[j], j, a.boys, a.out);
+    const long long o0 = bf.off[0];
+    if (staged) {
+      for (int i = threadIdx.x; i < total; i += IB2_TPB) {
+        const int j = st.order[i];
+        ib2_thread_pair<KIND>(bf, st.swp, st.cls[j], j, a.rows, st.out + (int)(bf.off[j] - o0));
+      }
+    } else {
+      for (int i = threadIdx.x; i < total; i += IB2_TPB) {
+        const int j = st.order[i];
+        ib2_thread_pair<KIND>(bf, st.swp, st.cls[j], j, a.rows, a.out + bf.off[j]);
+      }
     }
-    __syncthreads();  // this buffer and the sort arrays are reused
+    const int nout = staged ? (int)(bf.off[np - 1] - o0) + ib2_ncart(bf.la[np - 1]) * ib2_ncart(bf.lb[np - 1]) : 0;
+    __syncthreads();  // the inputs are read, the results staged
+    if (threadIdx.x == 0 && nxt < nfull) ib2_issue<KIND>(a, bf, nxt, mb);
+    for (int x = threadIdx.x; x < nout; x += IB2_TPB) a.out[o0 + x] = st.out[x];
+    __syncthreads();  // the staged results and the sort arrays are reused
   }
 }
 
@@ -721,6 +733,7 @@ struct TwoIdxDevice {
   bool ready = false;
   int nsm = 0;
   double* boys = nullptr;
+  double* rows = nullptr;
   Single* single = nullptr;
   double* single_out = nullptr;
   int* single_status = nullptr;
@@ -753,6 +766,10 @@ int twoidx_setup(TwoIdxDevice** out) {
     bool ok = cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
     ok = ok && cudaMemcpyToSymbol(ib2_boys, ib_boys_host_table, sizeof(ib_boys_host_table)) == cudaSuccess;
     ok = ok && cudaGetSymbolAddress((void**)&d.boys, ib2_boys) == cudaSuccess;
+    std::vector<double> rows;
+    ib_boys_rows_host(ib_boys_host_table, 4, rows);
+    ok = ok && cudaMemcpyToSymbol(ib2_rows, rows.data(), rows.size() * sizeof(double)) == cudaSuccess;
+    ok = ok && cudaGetSymbolAddress((void**)&d.rows, ib2_rows) == cudaSuccess;
     ok = ok && cudaGetSymbolAddress((void**)&d.single, ib2_single) == cudaSuccess;
     ok = ok && cudaGetSymbolAddress((void**)&d.single_out, ib2_single_out) == cudaSuccess;
     ok = ok && cudaGetSymbolAddress((void**)&d.single_status, ib2_single_status) == cudaSuccess;
@@ -895,6 +912,7 @@ void single_pair(int kind, double xa, const double* cA, int la, int na, int iski
   a.off = &d->single->off;
   a.out = d->single_out;
   a.boys = d->boys;
+  a.rows = d->rows;
   a.status = d->single_status;
   const int tot = na * nb;
   double res[28 * 28];
@@ -984,6 +1002,7 @@ int intception_b200_twoidx_batch(int kind, int n, int lmax, const double* xa, co
   a.off = off;
   a.out = out;
   a.boys = d->boys;
+  a.rows = d->rows;
   a.status = status;
   st = launch(kind, a, d->nsm, static_cast<cudaStream_t>(stream));
   if (st) return ib_runtime_set_status(st, "twoidx_batch: launch failed");

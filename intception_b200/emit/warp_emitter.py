@@ -343,7 +343,8 @@ class WarpEmitter(GroupEmitter):
         need = 2 * self.nacc() + self.in_flight() + 44
         best = 0
         for mi, minb in enumerate(MINB_VALUES):
-            if minb * self.block * need <= 65536 and minb * (self.smem + 1024) <= 227 * 1024:
+            per_part = -(-minb * self.block // 32 // 4)  # warps of an SM quarter, which shares 16384 registers
+            if 512 // per_part >= need and minb * (self.smem + 1024) <= 227 * 1024:
                 best = mi
         return best
 
