@@ -505,11 +505,6 @@ __global__ void __launch_bounds__(IB_GEN_BLOCK, MINB) ib_eri_generic(const IbLau
   __shared__ unsigned short eu[3 * IB_GEN_NCT];
   __shared__ unsigned char cp[(2 * IB_LMAX + 1) * (IB_LMAX + 1)];  // (f_x, f_y) pairs by f_x + f_y
   __shared__ int ticket;
-  ib_gen_tables(ct, em, eu);
-  if (threadIdx.x <= 2 * IB_LMAX)
-    for (int y = 0; y <= (int)threadIdx.x; ++y)
-      cp[threadIdx.x * (threadIdx.x + 1) / 2 + y] = (unsigned char)((threadIdx.x - y) | (y << 4));
-  __syncthreads();
   const int tid = threadIdx.x;
   int crank = 0;
   if constexpr (CS > 1) crank = (int)cg::this_cluster().block_rank();
@@ -527,6 +522,12 @@ __global__ void __launch_bounds__(IB_GEN_BLOCK, MINB) ib_eri_generic(const IbLau
     lb = a.ranges[wk.light_slot];
     nl = a.ranges[wk.light_slot + 1] - lb;
   }
+  if (nh + nl == 0) return;  // most redo lists: leave before the tables are built
+  ib_gen_tables(ct, em, eu);
+  if (threadIdx.x <= 2 * IB_LMAX)
+    for (int y = 0; y <= (int)threadIdx.x; ++y)
+      cp[threadIdx.x * (threadIdx.x + 1) / 2 + y] = (unsigned char)((threadIdx.x - y) | (y << 4));
+  __syncthreads();
   // item t of the heavy list (t < nh), then of the light list
   auto item = [&](int t) -> int {
     if (t < nh) return wk.redo ? a.redo[2 + t] : hb + t;

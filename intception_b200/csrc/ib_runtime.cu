@@ -134,10 +134,12 @@ struct Context {
   int slice_cap[IB_NCLASS] = {};  // per class: cap on lane groups per quartet (0: no cap; INTCEPTION_B200_MAX_SLICES)
   // INTCEPTION_B200_SLICE_BOOST: slices chosen as if the grid had this many
   // times its lane groups.  The class kernels of a batch run concurrently and
-  // their quartets differ widely in length; measured on the l <= 2 workload,
-  // 4 shortens the last, thinly occupied waves (screened step -17 %, full
-  // FP64 step -5 %) and 8 is slower again.
-  int slice_boost = 4;
+  // their quartets differ widely in length, so more slices than fill the grid
+  // shorten the thinly occupied last waves; each slice costs its own chunk
+  // remainders.  Boost 1 / 2 / 3 / 4 / 8: screened l <= 2 step 1.50 / 1.37 /
+  // 1.48 / 1.57 / 1.95 ms, 200-atom lattice sample 5.48 / 5.55 / 5.59 / 5.77 /
+  // 6.36 ms, the full l <= 2 FP64 step 8.06-8.09 ms with any of them.
+  int slice_boost = 2;
   double prim_tol = 0.0;  // batch entries: primitive-quartet screening tolerance (0: exact zeros only)
   // class kernels: quartets whose HRR rounding-error estimate (IB_HRR_ERR_COEF
   // x the largest weighted contracted element) exceeds this are recomputed by
@@ -671,6 +673,18 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, int nq, bool fp64_pr
   for (size_t i = 0; i < c->classes.size(); ++i)
     if (c->lmax_of[i] <= lmax)
       nuse += (fp64_present ? 1 : 0) + (fp32_present && c->kind_h[c->classes[i]] == 2 ? 2 : 0);
+  // fewer for large batches: a class kernel that runs by itself is up to a
+  // tenth faster than one sharing its SMs (their instruction caches), and the
+  // overlap only pays for the launches' tails.  27-atom J/K energy chunks
+  // (2.1e6 quartets) 53.0 ms in all with 40, 4 or 2 streams, 48.3 with one;
+  // 200-atom lattice sample (1e6 quartets, 65 classes) 5.56 ms with 40, 5.37
+  // with 4, 5.77 with one; screened, where few quartets are left, 1.39 / 1.35 /
+  // 2.04 ms with 40, 8 and one; the l <= 4 sample (46 quartets a class) 26 / 41
+  // / 84 ms with 40, 4 and one.
+  if (nq >= 3 << 19 && !zf)
+    nuse = 1;
+  else if (nq / nuse >= 8192)
+    nuse = std::min(nuse, zf ? 8 : 4);
   nuse = std::max(1, std::min(nuse, c->nside));
   IB_CUDA(cudaEventRecord(c->fork, s));
   for (int i = 0; i < nuse; ++i) IB_CUDA(cudaStreamWaitEvent(c->side[i], c->fork, 0));
@@ -969,10 +983,6 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
     a.redo_cap = nblk;
     a.hrr_tol = c->hrr_tol;
     c->table[cidx].launch(vt, grid, s, a);
-    // a class without an HRR has no check that could fill the list
-    if (a.hrr_tol > 0.0 && (lperm[1] > 0 || lperm[3] > 0))
-      IB_CUDA(redo_launch(c, s, a, false, std::max(std::max(sh[0].l, sh[1].l), std::max(sh[2].l, sh[3].l)),
-                          nullptr));
   } else {
     const long long slice = generic_slice(std::max(std::max(sh[0].l, sh[1].l), std::max(sh[2].l, sh[3].l)));
     long long nb = std::min<long long>({(long long)nblk, (long long)ib_generic_bps() * c->nsm,
@@ -983,26 +993,36 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
                               slice));
   }
   IB_CUDA(cudaGetLastError());
-  if (sph) {
-    IbXform x;
-    for (int i = 0; i < 4; ++i) {
-      x.T[i] = reinterpret_cast<const double*>(d + o_T[i]);
-      x.l[i] = sh[i].l;
-      x.n[i] = sh[i].n;
+  auto finish = [&]() -> cudaError_t {
+    if (sph) {
+      IbXform x;
+      for (int i = 0; i < 4; ++i) {
+        x.T[i] = reinterpret_cast<const double*>(d + o_T[i]);
+        x.l[i] = sh[i].l;
+        x.n[i] = sh[i].n;
+      }
+      x.nblk = nblk;
+      x.cart_block = cart_block;
+      x.res_block = res_block;
+      ib_transform_blocks<<<nblk, 128, 0, s>>>(x, c->d_cart.as<double>(), dres, c->d_res.as<double>());
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
     }
-    x.nblk = nblk;
-    x.cart_block = cart_block;
-    x.res_block = res_block;
-    ib_transform_blocks<<<nblk, 128, 0, s>>>(x, c->d_cart.as<double>(), dres, c->d_res.as<double>());
-    IB_CUDA(cudaGetLastError());
-  }
-  // control words, status word and result in one copy
-  IB_CUDA(cudaMemcpyAsync(c->h_res.p, d + o_ctl, total - o_ctl, cudaMemcpyDeviceToHost, s));
-  IB_CUDA(cudaStreamSynchronize(s));
+    // control words, status word and result in one copy
+    const cudaError_t e = cudaMemcpyAsync(c->h_res.p, d + o_ctl, total - o_ctl, cudaMemcpyDeviceToHost, s);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s);
+  };
+  IB_CUDA(finish());
   const char* hr = static_cast<const char*>(c->h_res.p);
+  c->host_redo = reinterpret_cast<const int*>(hr)[2] + reinterpret_cast<const int*>(hr)[3];
+  if (c->host_redo > 0) {
+    // the HRR check listed quartets: recompute them, then the result again (few
+    // calls need it, and a launch that finds an empty list costs 5 us)
+    IB_CUDA(redo_launch(c, s, a, false, std::max(std::max(sh[0].l, sh[1].l), std::max(sh[2].l, sh[3].l)), nullptr));
+    IB_CUDA(finish());
+  }
   const int hstatus = *reinterpret_cast<const int*>(hr + (o_status - o_ctl));
   c->host_status = hstatus;
-  c->host_redo = reinterpret_cast<const int*>(hr)[2] + reinterpret_cast<const int*>(hr)[3];
   if (hstatus) return set_status(hstatus, "device kernel reported status " + std::to_string(hstatus));
   // place the compact result at the caller's strides (the emitted code's final
   // copy loop, contracted_general.py:1808-1876)

@@ -664,16 +664,17 @@ __global__ void __launch_bounds__(IB2_TPB, 2) ib2_thread_kernel(const Ib2Args a)
     __syncthreads();
     const int total = st.start[kClasses];
     const long long o0 = bf.off[0];
-    if (staged) {
-      for (int i = threadIdx.x; i < total; i += IB2_TPB) {
-        const int j = st.order[i];
+    // units of 32 pairs in ascending class (cost) order; warp w takes unit w and
+    // unit IB2_WR - 1 - w, so that the warps' shares are alike at the barrier
+#pragma unroll 1
+    for (int q = 0; q < kRounds; ++q) {
+      const int i = 32 * (q & 1 ? (q + 1) * (IB2_TPB / 32) - 1 - warp : q * (IB2_TPB / 32) + warp) + lane;
+      if (i >= total) continue;
+      const int j = st.order[i];
+      if (staged)
         ib2_thread_pair<KIND>(bf, st.swp, st.cls[j], j, a.rows, st.out + (int)(bf.off[j] - o0));
-      }
-    } else {
-      for (int i = threadIdx.x; i < total; i += IB2_TPB) {
-        const int j = st.order[i];
+      else
         ib2_thread_pair<KIND>(bf, st.swp, st.cls[j], j, a.rows, a.out + bf.off[j]);
-      }
     }
     const int nout = staged ? (int)(bf.off[np - 1] - o0) + ib2_ncart(bf.la[np - 1]) * ib2_ncart(bf.lb[np - 1]) : 0;
     __syncthreads();  // the inputs are read, the results staged
