@@ -901,6 +901,29 @@ __device__ __forceinline__ void ib_rys_setup(const double* __restrict__ pab, con
   o[11 * 32] = q.fd;
 }
 
+// The same for the kernels by rotated axes: per axis d (4 d + 0..3) P_d - A_d,
+// W_d - P_d, Q_d - C_d, W_d - Q_d, then 1/2zeta, rho/2zeta^2, 1/2eta,
+// rho/2eta^2, 1/2(zeta+eta); tp: the Boys argument and, 32 further, the prefactor.
+__device__ __forceinline__ void ib_rot_setup(const double* __restrict__ pab, const double* __restrict__ pcd,
+                                             const IbQuartet& g, double* __restrict__ o, double* __restrict__ tp) {
+  IbGeom q;
+  ib_geometry(pab, pcd, g, q);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    o[(4 * d + 0) * 32] = -q.fb * g.AB[d];
+    o[(4 * d + 1) * 32] = -q.roz * q.PQ[d];
+    o[(4 * d + 2) * 32] = -q.fd * g.CD[d];
+    o[(4 * d + 3) * 32] = q.roe * q.PQ[d];
+  }
+  o[12 * 32] = 0.5 * q.oz;
+  o[13 * 32] = 0.5 * q.oz * q.roz;
+  o[14 * 32] = 0.5 * q.oe;
+  o[15 * 32] = 0.5 * q.oe * q.roe;
+  o[16 * 32] = 0.5 * q.ozpe;
+  tp[0] = q.T;
+  tp[32] = q.pref;
+}
+
 // Rows of ib_boys_row for L = 0..lmax from the full table (rows of IB_BOYS_NCOL values F_n(T_i)).
 inline void ib_boys_rows_host(const double* table, int lmax, std::vector<double>& rows) {
   rows.assign((size_t)(lmax + 1) * IB_BOYS_NPTS * 8, 0.0);

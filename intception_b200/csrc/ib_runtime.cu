@@ -163,6 +163,7 @@ struct Context {
   int redo_groups = 1, redo_stride = 2;
   DevBuf tickets;  // kTickets ints: the generic kernel's ticket pairs (zeroed by every dispatch)
   DevBuf kind;                                              // per class: 0 generic, 1 FP64, 2 FP64+FP32
+  int fp32_classes = 0;        // classes with kind 2
   int kind_h[IB_NCLASS] = {};  // host copy of kind: 2 where the class has FP32 kernels and the FP32 tier uses them
   DevBuf d_stage, d_cart, d_res;
   HostBuf h_stage, h_res;
@@ -585,6 +586,7 @@ int get_context(Context** out) {
       if (!c->table[cid].launch) continue;
       kind[cid] = (c->table[cid].kind == 2 && ib_tuned_fp32[cid]) ? 2 : 1;
       c->kind_h[cid] = kind[cid];
+      c->fp32_classes += kind[cid] == 2;
       for (int v = 0; v < 4 * IB_NMINB; ++v) c->occ[cid][v] = std::max(1, c->table[cid].occupancy(v));
       for (int v = 0; v < 4; ++v) c->minb_idx[cid][v] = std::min(std::max(ib_tuned_minb[cid][v], 0), IB_NMINB - 1);
       c->slice_cap[cid] = ib_tuned_slice_cap[cid];
@@ -1199,6 +1201,8 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   if ((precision == IB_PREC_MIXED || skip_below > 0.0) && !bounds)
     return set_status(IB_ERR_ARG, "eri_batch: mixed precision and screening need bounds");
   if (nq == 0) return set_status(IB_OK, "");
+  // the FP32 tier with no FP32 class kernel in use is the FP64 path
+  if (c->fp32_classes == 0) precision = IB_PREC_FP64;
   if (nq <= kSmallBatch && basis->lmax <= ib_lmax_emitted && precision == IB_PREC_FP64 && c->hrr_tol > 0.0)
     return small_batch(c, basis, quartets, out_off, nq, spherical, skip_below > 0.0 ? bounds : nullptr, skip_below, out,
                        s, nl, screen_prims);
@@ -1643,6 +1647,7 @@ int intception_b200_set_class_fp32(int cid, int on) {
     const int want = on < 0 ? ib_tuned_fp32[k] : on;
     c->kind_h[k] = (c->table[k].kind == 2 && want) ? 2 : 1;
   }
+  c->fp32_classes = (int)std::count(c->kind_h, c->kind_h + IB_NCLASS, 2);
   IB_CUDA(cudaDeviceSynchronize());
   IB_CUDA(cudaMemcpy(c->kind.p, c->kind_h, IB_NCLASS * sizeof(int), cudaMemcpyHostToDevice));
   return set_status(IB_OK, "");

@@ -412,9 +412,18 @@ def thread_class(c):
 
 THREAD_TARGETS = 54
 
+# classes on the rotated-axes kernel (warp_emitter.RotationEmitter); ns per
+# quartet with 2D tables and with rotation, K 1..6 in a 30-bohr box: (pp|pp) 9.0
+# and 8.3 (8 bohr, K = 3: 11.4 and 10.2), (dd|ps) 14.2 and 11.5, (fd|ps) 22.7 and
+# 20.2.  The other ps, pp and ds kets are level or slower: their lanes run out
+# of registers ((dp|pp) 15.7 and 16.6) or the lane-per-primitive kernel serves them.
+ROTATED = {(1, 1, 1, 1), (2, 2, 1, 0), (3, 2, 1, 0)}
+
 
 def fp64_emitter(c):
-    from .warp_emitter import RysEmitter, ThreadEmitter
+    from .warp_emitter import RotationEmitter, RysEmitter, ThreadEmitter
+    if c in ROTATED:
+        return RotationEmitter(*c)
     return ThreadEmitter(*c) if thread_class(c) else RysEmitter(*c)
 
 
@@ -564,7 +573,6 @@ def emit_all(outdir, lmax=LMAX_EMIT, ngroups=24):
         for tag, ent in tun.get('classes', {}).items():
             cid = class_id(*(int(ch) for ch in tag))
             minb[cid] = [int(x) for x in ent.get('minb', [0, 0, 0, 0])]
-            minb[cid][:2] = ent.get('warp_minb', [budget[cid]] * 2)
             scap[cid] = int(ent.get('slice_cap', DEFAULT_SLICE_CAP))
             fp32on[cid] = 1 if ent.get('fp32', True) else 0
     disp.append('extern const int ib_tuned_minb[%d][4] = {%s};'

@@ -68,6 +68,7 @@ class WarpEmitter(GroupEmitter):
     slices, the HRR check and the epilogue (GroupEmitter's)."""
 
     G = 32  # lanes per group
+    chunk = CHUNK
 
     def __init__(self, la, lb, lc, ld):
         # no GroupEmitter layout: only its epilogue pieces are used
@@ -163,7 +164,7 @@ class WarpEmitter(GroupEmitter):
         A('      const float rn1 = 1.0f / (float)max(nl1, 1);')
         # chunks of the unscreened loop: as even over the slices as the 2D step allows
         if NB > 1:
-            A('      const int ch = min(%d, ((npl + W - 1) / W + %d) / %d * %d);' % (CHUNK, NB - 1, NB, NB))
+            A('      const int ch = min(%d, ((npl + W - 1) / W + %d) / %d * %d);' % (self.chunk, NB - 1, NB, NB))
         else:
             A('      const int ch = min(%d, max((npl + W - 1) / W, 1));' % CHUNK)
         A('      int q0 = pre ? 32 * w : ch * w, left = 0;')
@@ -172,7 +173,7 @@ class WarpEmitter(GroupEmitter):
         A('        if (pre) {')
         # survivors of the screen, collected by the group's first warp
         A('          if (j < 32) {')
-        A('            while (left < %d && q0 < npl) {' % CHUNK)
+        A('            while (left < %d && q0 < npl) {' % self.chunk)
         A('              const int u = q0 + j, ua = (int)(((float)u + 0.5f) * rn1), uc = u - ua * nl1;')
         A('              const bool ok = u < npl && !ib_quartet_negligible(lst, ua, uc, a.prim_tol);')
         A('              const unsigned bal = __ballot_sync(0xffffffffu, ok);')
@@ -184,7 +185,7 @@ class WarpEmitter(GroupEmitter):
             A('            if (j == 0) *qcnt = left;')
         A('          }')
         A('          %s;' % sync)
-        A('          n = min(%s, %d);' % ('*qcnt' if wide else 'left', CHUNK))
+        A('          n = min(%s, %d);' % ('*qcnt' if wide else 'left', self.chunk))
         A('          if (n == 0) break;  // uniform over the group')
         A('          if (j < n) { qa = que[j] & 255; qc = que[j] >> 8; }')
         A('        } else {')
@@ -676,4 +677,151 @@ class ThreadEmitter(WarpEmitter):
             k = '%d + j' % k0 if k0 else 'j'
             L.append('      sb[(%s) / %d * %d + (%s) %% %d] = s0 + s1;' % (k, nf, nfp, k, nf))
             L.append('    }')
+        return L
+
+
+class RotationEmitter(WarpEmitter):
+    """Rys kernel without 2D tables: three lanes per primitive quartet, ten
+    primitive quartets per warp.  The targets of an s-p, p-p or s-d lane side
+    fall into orbits of the cyclic axis permutation (x, xx, xy stand for all
+    nine of levels 1 and 2), so lane k evaluates one representative of each
+    with its axes rotated by k: the same instructions on every lane, every 2D
+    integral in the lane's registers, no step between roots and products."""
+
+    kind = 'rot'
+    ORBITS = {(1, 0): ((1, 0, 0),), (1, 1): ((1, 0, 0), (2, 0, 0), (1, 1, 0)), (2, 0): ((2, 0, 0), (1, 1, 0))}
+    NB = 10
+    NTAB = 5      # partial tables: the second five primitive quartets add to the first five's
+    chunk = 30    # three full passes
+
+    @classmethod
+    def fits(cls, la, lb, lc, ld):
+        return (lc, ld) in cls.ORBITS
+
+    def __init__(self, la, lb, lc, ld):
+        super().__init__(la, lb, lc, ld)
+        self.N = self.L // 2 + 1
+        self.orbits = self.ORBITS[lc, ld]
+        self.ctargets = comps_range(la, self.E)
+        self.stargets = comps_range(lc, self.F)
+        self.n = len(self.orbits) * len(self.ctargets)
+
+    def in_flight(self):
+        sx, sy = max(o[0] for o in self.orbits), max(o[1] for o in self.orbits)
+        return 2 * ((self.E + 1) * (sx + sy + 3) + 12) + 16
+
+    def nacc(self):
+        return self.n
+
+    def layout(self, tbl):
+        self.o_uw = 17 * CHUNK
+        self.o_tp = self.o_uw + 2 * self.N * CHUNK
+        return max(self.o_tp + 2 * CHUNK, self.NTAB * tbl), self.NTAB
+
+    def table_offset(self, orbit, c, k):
+        """Offset in a contracted table of the local target (orbit, c) of lane k."""
+        turn = lambda v: tuple(v[(i - k) % 3] for i in range(3))  # noqa: E731  local axis i is axis (k + i) mod 3
+        nf = len(self.stargets)
+        return self.ctargets.index(turn(c)) * (nf if nf % 2 else nf + 1) + self.stargets.index(turn(orbit))
+
+    def constants(self):
+        words = []
+        for o in self.orbits:
+            for c in self.ctargets:
+                w = [self.table_offset(o, c, k) for k in range(3)]
+                assert max(w) < 1024
+                words.append(w[0] | (w[1] << 10) | (w[2] << 20))
+        return ['__constant__ unsigned ib_rot_%s_at[%d] = {%s};' % (self.tag, self.n, ', '.join('%du' % w for w in words))]
+
+    def describe(self):
+        return 'Rys quadrature by rotated axes: %d roots, %d accumulators' % (self.N, self.n)
+
+    def prologue(self):
+        L = ['  const int pg = j / 3, rk = j % 3;  // primitive quartet of the pass, rotation',
+             '  const bool own = pg < 10;']
+        for i, d in enumerate('xyz'):
+            L.append('  const double* __restrict__ f%s = sb + pg + ((rk + %d) %% 3) * %d;' % (d, i, 4 * CHUNK))
+        return L
+
+    def chunk_body(self, sync):
+        N, C = self.N, self.E
+        src = []
+        A = src.append
+        A('        if (j < n) ib_rot_setup(pd + 4 * qa, pd + 4 * (%d + qc), g, sb + j, sb + %d + j);' % (PAIR_TILE, self.o_tp))
+        A('        %s;' % sync)
+        A('        for (int x = j; x < n * %d; x += 32) {' % N)
+        A('          const int u = x / %d, rt = x - u * %d;' % (N, N))
+        A('          ib_rys_root<%d>(a.rys_tab, sb[%d + u], sb[%d + u], rt, sb + %d + 2 * x);'
+          % (N, self.o_tp, self.o_tp + CHUNK, self.o_uw))
+        A('        }')
+        A('        %s;' % sync)
+        A('        for (int s0 = 0; s0 < n; s0 += 10) {')
+        A('          if (!(own && s0 + pg < n)) continue;')
+        for d in 'xyz':
+            A('          const double c%s0 = f%s[s0], c%s1 = f%s[s0 + %d], l%s0 = f%s[s0 + %d], l%s1 = f%s[s0 + %d];'
+              % (d, d, d, d, CHUNK, d, d, 2 * CHUNK, d, d, 3 * CHUNK))
+            A('          (void)l%s0; (void)l%s1;' % (d, d))
+        A('          const double* __restrict__ fb = sb + %d + s0 + pg;' % (12 * CHUNK))
+        A('          const double b0 = fb[0], b1 = fb[%d], e0 = fb[%d], e1 = fb[%d], h = fb[%d];'
+          % (CHUNK, 2 * CHUNK, 3 * CHUNK, 4 * CHUNK))
+        A('          (void)e0; (void)e1;')
+        A('          const double2* __restrict__ uwp = reinterpret_cast<const double2*>(sb + %d) + (s0 + pg) * %d;' % (self.o_uw, N))
+        A('#pragma unroll 1')
+        A('          for (int rt = 0; rt < %d; ++rt) {' % N)
+        A('            const double u = uwp[rt].x, wt = uwp[rt].y;')
+        A('            const double CB = fma(-u, b1, b0), LB = fma(-u, e1, e0), B00 = u * h;  // chain, lane side, mixed')
+        A('            (void)CB; (void)LB; (void)B00;')
+        smax = (max(o[0] for o in self.orbits), max(o[1] for o in self.orbits), 0)
+        val = {}
+        for i, d in enumerate('xyz'):
+            A('            const double C%s = fma(u, c%s1, c%s0);' % (d, d, d))
+            if smax[i]:
+                A('            const double L%s = fma(u, l%s1, l%s0);' % (d, d, d))
+
+            def mul(k, a, b):  # k * a * b, with 1 dropped
+                t = [x for x in ('%d.0' % k if k > 1 else None, a, b if b != '1.0' else None) if x]
+                return ' * '.join(t)
+
+            def put(c, sv, terms):
+                # terms: (coefficient, factor, value) summed as FMAs, the last first
+                e = mul(*terms[-1])
+                for k, a, b in reversed(terms[:-1]):
+                    e = 'fma(%s, %s, %s)' % (mul(k, a, '1.0'), b, e) if b != '1.0' else '%s + %s' % (mul(k, a, '1.0'), e)
+                name = '%s%d_%d' % (d, c, sv)
+                A('            const double %s = %s;' % (name, e))
+                val[i, c, sv] = name
+            val[i, 0, 0] = 'wt' if i == 2 else '1.0'
+            for c in range(C):
+                put(c + 1, 0, [(1, 'C' + d, val[i, c, 0])] + ([(c, 'CB', val[i, c - 1, 0])] if c else []))
+            for sv in range(smax[i]):
+                for c in range(C + 1):
+                    put(c, sv + 1, [(1, 'L' + d, val[i, c, sv])] + ([(sv, 'LB', val[i, c, sv - 1])] if sv else []) +
+                        ([(c, 'B00', val[i, c - 1, sv])] if c else []))
+        yz = {}
+        for o, orb in enumerate(self.orbits):
+            for t, c in enumerate(self.ctargets):
+                key = (c[1], orb[1], c[2])
+                if key not in yz:
+                    y, z = val[1, c[1], orb[1]], val[2, c[2], 0]
+                    if y == '1.0':
+                        yz[key] = z
+                    else:
+                        yz[key] = 'p%d_%d_%d' % key
+                        A('            const double %s = %s * %s;' % (yz[key], y, z))
+                A('            acc[%d] = fma(%s, %s, acc[%d]);'
+                  % (o * len(self.ctargets) + t, val[0, c[0], orb[0]], yz[key], o * len(self.ctargets) + t))
+        A('          }')
+        A('        }')
+        return src
+
+    def write_tables(self, nfp, tbl):
+        L = ['    double* __restrict__ mine = sb + (pg < %d ? pg : pg - %d) * %d;' % (self.NTAB, self.NTAB, tbl)]
+        for half in (0, 1):
+            L.append('    if (own && pg %s %d) {' % ('>=' if half else '<', self.NTAB))
+            for k in range(self.n):
+                L.append('      mine[(ib_rot_%s_at[%d] >> (10 * rk)) & 1023u] %s acc[%d];'
+                         % (self.tag, k, '+=' if half else '=', k))
+            L.append('    }')
+            if not half:
+                L.append('    __syncwarp();')
         return L
