@@ -147,7 +147,7 @@ struct Context {
   double hrr_tol = 1e-13;
   cudaStream_t side[kNSideMax] = {};
   cudaEvent_t fork = nullptr, join[kNSideMax] = {};
-  DevBuf boys_tab, rys_tab, boys_row, sph, keys, vals, keys2, vals2, items, ranges, status, cub_tmp, scratch;
+  DevBuf boys_tab, rys_tab, boys_row, sph, keys, vals, keys2, vals2, items, ranges, cub_tmp, scratch;
   DevBuf counters;  // per class kernel launch of a batch: the next quartet (FP64, FP32, FP64 recheck passes)
   DevBuf sw_quartets, sw_sizes, sw_off, sw_tmp, sw_blocks;  // Schwarz-bound work buffers
   std::vector<int> classes;  // emitted class ids, the heaviest first (descending id)
@@ -156,6 +156,7 @@ struct Context {
   int flags_nq = 0;  // its quartet count (flags beyond it are stale)
   // the small-batch kernel's control words and items, sized once for the largest such batch
   DevBuf small_ctl, small_items;
+  int* status = nullptr;  // status word of every batch, whichever path it takes (the first control word)
   const int* last_status = nullptr;  // status word and redo list of the last batch
   const int* last_redo = nullptr;    // (null after a drop-in call: the host copies)
   int host_status = 0, host_redo = 0;
@@ -572,12 +573,12 @@ int get_context(Context** out) {
     IB_CUDA(cudaMemcpy(c->sph.p, sph.data(), sph.size() * sizeof(double), cudaMemcpyHostToDevice));
     IB_CUDA(c->ranges.ensure(kNRanges * sizeof(int)));
     IB_CUDA(c->counters.ensure((kNCounters + 1) * sizeof(int)));  // + the drop-in's own
-    IB_CUDA(c->status.ensure(sizeof(int)));
-    IB_CUDA(cudaMemset(c->status.p, 0, sizeof(int)));
     IB_CUDA(c->tickets.ensure(kTickets * sizeof(int)));
     IB_CUDA(c->small_ctl.ensure((18 + 2 * (size_t)kSmallBatch) * sizeof(int)));
+    c->status = c->small_ctl.as<int>();
+    IB_CUDA(cudaMemset(c->status, 0, sizeof(int)));
+    c->last_status = c->status;
     IB_CUDA(c->small_items.ensure((size_t)kSmallBatch * sizeof(IbItem)));
-    c->last_status = c->status.as<int>();
     IB_CUDA(ib_small_prepare_cart());
     IB_CUDA(ib_small_prepare_sph());
     ib_register_emitted_classes(c->table);
@@ -615,7 +616,7 @@ IbLaunch base_launch(Context* c) {
   a.rys_tab = c->rys_tab.as<double>();
   a.boys_row = c->boys_row.as<double>();
   a.sph = c->sph.as<double>();
-  a.status = c->status.as<int>();
+  a.status = c->status;
   a.slice_boost = c->slice_boost;
   a.split_min = ib_generic_split_min();
   return a;
@@ -1221,9 +1222,9 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   c->redo_stride = nq + 2;
   IB_CUDA(c->redo.ensure((size_t)c->redo_groups * (nq + 2) * sizeof(int)));
   c->flags_nq = nq;
-  c->last_status = c->status.as<int>();
+  c->last_status = c->status;
   c->last_redo = c->redo.as<int>();
-  IB_CUDA(cudaMemsetAsync(c->status.p, 0, sizeof(int), s));
+  IB_CUDA(cudaMemsetAsync(c->status, 0, sizeof(int), s));
   const IbZeroed zeroed = {c->ranges.as<int>(), c->counters.as<int>(), c->tickets.as<int>(), c->redo.as<int>(),
                            c->flags.as<int>(), kNRanges, kNCounters, kTickets, c->redo_groups, c->redo_stride};
   const int grid = std::min((nq + 255) / 256, c->nsm * 16);
@@ -1233,7 +1234,7 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
                                    use_bounds ? bounds : nullptr, skip_below, fp32_below,
                                    precision == IB_PREC_MIXED ? 1 : 0, c->kind.as<int>(), c->hrr_tol > 0.0 ? 0 : 1,
                                    ib_generic_split_min(), c->keys.as<unsigned>(),
-                                   c->vals.as<int>(), c->status.as<int>(), zeroed);
+                                   c->vals.as<int>(), c->status, zeroed);
   ++*nl;
   IB_CUDA(cudaGetLastError());
   IB_CUDA(cub::DeviceRadixSort::SortPairs(c->cub_tmp.p, tmp_bytes, c->keys.as<unsigned>(), c->keys2.as<unsigned>(),
@@ -1480,6 +1481,9 @@ struct IbGraph {
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   int launches;
+  int nq;
+  bool small;  // captured the small-batch kernel: its redo list lies in the control words
+  int flags_nq, redo_groups, redo_stride;
 };
 
 int intception_b200_eri_graph_create(const intception_b200_basis* basis, const int* quartets, const long long* out_off,
@@ -1502,7 +1506,8 @@ int intception_b200_eri_graph_create(const intception_b200_basis* basis, const i
     return st;
   }
   IB_CUDA(cudaStreamSynchronize(s));
-  IbGraph* g = new IbGraph{c, nullptr, nullptr, 0};
+  IbGraph* g = new IbGraph{c, nullptr, nullptr, 0, nq, c->last_redo != c->redo.as<int>(), c->flags_nq, c->redo_groups,
+                           c->redo_stride};
   IB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   nl = 0;
   st = batch_impl(c, basis, quartets, out_off, nq, spherical, precision, bounds, skip_below, fp32_below, mixed_tol,
@@ -1531,6 +1536,14 @@ int intception_b200_eri_graph_launch(void* handle, void* stream) {
   IbGraph* g = static_cast<IbGraph*>(handle);
   if (!g) return set_status(IB_ERR_ARG, "graph_launch: null handle");
   tl_launches = g->launches;
+  // the status and redo queries refer to this batch from here on
+  Context* c = g->ctx;
+  std::lock_guard<std::mutex> lk(c->mu);
+  c->last_status = c->status;
+  c->last_redo = g->small ? c->status + 16 + g->nq : c->redo.as<int>();
+  c->flags_nq = g->flags_nq;
+  c->redo_groups = g->redo_groups;
+  c->redo_stride = g->redo_stride;
   IB_CUDA(cudaGraphLaunch(g->exec, static_cast<cudaStream_t>(stream)));
   return set_status(IB_OK, "");
 }

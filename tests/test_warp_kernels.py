@@ -85,3 +85,23 @@ def test_pair_counts_around_the_tile(ls, ks):
     out = eng.compute().cpu().numpy()
     eri.set_prim_tol(0.0)
     assert np.abs(out - ref).max() <= tolerance(ref) + np.prod(np.array(ks, float)) * 1e-18
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('nq', [8, 400])
+@pytest.mark.parametrize('between', [8, 400])
+def test_status_after_graph_replay(nq, between):
+    """The status read after a replay is the replayed batch's, on the small-batch
+    kernel and on the pipeline, whichever of them ran in between."""
+    import torch
+    bad = eri.EriEngine(basis.independent_quartet_batch(5, nq, [2], [1, 2], 0.1, 60.0, 6.0, True))
+    bad._basis.lmax = 1  # declared lmax below the shells' l
+    good = eri.EriEngine(basis.independent_quartet_batch(6, between, [0, 1, 2], [1, 2], 0.1, 60.0, 6.0, True))
+    g = bad.graph(torch.empty(bad.out_size, dtype=torch.float64, device='cuda'))
+    good.compute()
+    assert good.device_status() == 0
+    g.launch()
+    assert bad.device_status() == eri.IB_ERR_ARG
+    good.compute()
+    assert good.device_status() == 0
+    g.close()
