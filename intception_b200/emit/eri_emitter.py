@@ -34,9 +34,7 @@ sys.path.insert(0, os.path.dirname(os.path.dirname(HERE)))
 
 from intception_b200.basis import sph_matrix  # noqa: E402
 
-LMAX_EMIT = 2  # classes with every l <= LMAX_EMIT get an unrolled kernel
-# classes kept on the one-thread-per-quartet kernel (everything else whose
-# smaller side fits a warp uses the lane-group kernel of group_emitter.py)
+LMAX_EMIT = 2  # classes with every l <= LMAX_EMIT are built for every register budget and in the small-batch kernels
 
 DIRS = 'xyz'
 NPAIR_TOTAL = 7 * 8 // 2                       # shell pairs with l <= 6 (IB_NPAIR)
@@ -325,71 +323,15 @@ class Emitter:
             lines.append('    o[%s] = %s[%d];' % (offs or '0', cur, flat))
         return lines
 
-    # ------------------------------------------------------------ kernel
-    def kernel(self):
-        L = self.L
-        vrr = self.emit_vrr()
-        hrr = self.emit_hrr()
-        st_cart = self.emit_store(False)
-        st_sph = self.emit_store(True)
-        sph_flops = self.sph_flops
-        nacc = len(self.E) * len(self.F)
-        t = self.tag
-        cid = class_id(self.la, self.lb, self.lc, self.ld)
-        src = []
-        src.append('// ---- class (%d%d|%d%d): %d VRR nodes, %d VRR flops/primitive quartet, %d HRR flops'
-                   % (self.la, self.lb, self.lc, self.ld, self.nvar, self.flops, self.hrr_flops))
-        src.append('template <typename R, bool SPH>')
-        src.append('__global__ void __launch_bounds__(IB_BLOCK) ib_eri_%s(const IbLaunch a) {' % t)
-        src.append('  const int beg = a.ranges[2 * %d], end = a.ranges[2 * %d + 1];' % (cid, cid))
-        src.append('  if (beg + (int)(blockIdx.x * blockDim.x) >= end) return;  // block-uniform')
-        src.append('  for (int p = beg + blockIdx.x * blockDim.x + threadIdx.x; p < end; p += gridDim.x * blockDim.x) {')
-        src.append('    IbQuartet g;')
-        src.append('    ib_load_quartet(a, p, g);')
-        src.append('    double acc[%d];' % nacc)
-        src.append('#pragma unroll')
-        src.append('    for (int k = 0; k < %d; ++k) acc[k] = 0.0;' % nacc)
-        src.append('    for (int ia = 0; ia < g.k[0]; ++ia)')
-        src.append('    for (int ib = 0; ib < g.k[1]; ++ib) {')
-        src.append('      IbBraPair bp;')
-        src.append('      ib_bra_pair<sizeof(R) == 4>(a, g, ia, ib, bp);')
-        src.append('      if (bp.K == 0.0) continue;')
-        src.append('      for (int ic = 0; ic < g.k[2]; ++ic)')
-        src.append('      for (int id = 0; id < g.k[3]; ++id) {')
-        src.append('      IbPrimQuartet<R> pq;')
-        src.append('      double F[%d];' % (L + 1))
-        src.append('      if (!ib_prim_quartet<R, %d>(a, g, bp, ic, id, a.boys_tab, F, pq)) continue;' % L)
-        for m in range(L + 1):
-            src.append('      const R s%d = (R)F[%d];' % (m, m))
-        src.append('      const R PAx = pq.PA[0], PAy = pq.PA[1], PAz = pq.PA[2];')
-        src.append('      const R WPx = pq.WP[0], WPy = pq.WP[1], WPz = pq.WP[2];')
-        src.append('      const R QCx = pq.QC[0], QCy = pq.QC[1], QCz = pq.QC[2];')
-        src.append('      const R WQx = pq.WQ[0], WQy = pq.WQ[1], WQz = pq.WQ[2];')
-        src.append('      const R o2z = pq.o2z, roz = pq.roz, o2e = pq.o2e, roe = pq.roe, o2zpe = pq.o2zpe;')
-        src.append('      (void)PAx; (void)PAy; (void)PAz; (void)WPx; (void)WPy; (void)WPz;')
-        src.append('      (void)QCx; (void)QCy; (void)QCz; (void)WQx; (void)WQy; (void)WQz;')
-        src.append('      (void)o2z; (void)roz; (void)o2e; (void)roe; (void)o2zpe;')
-        src += vrr
-        src.append('      }')
-        src.append('    }')
-        src.append('    const double ABx = g.AB[0], ABy = g.AB[1], ABz = g.AB[2];')
-        src.append('    const double CDx = g.CD[0], CDy = g.CD[1], CDz = g.CD[2];')
-        src.append('    (void)ABx; (void)ABy; (void)ABz; (void)CDx; (void)CDy; (void)CDz;')
-        src += hrr
-        src.append('    double* __restrict__ o = a.out + g.off;')
-        src.append('    const int st0 = g.st[0], st1 = g.st[1], st2 = g.st[2], st3 = g.st[3];')
-        src.append('    (void)st0; (void)st1; (void)st2; (void)st3;')
-        src.append('    if (SPH) {')
-        src += ['  ' + s for s in st_sph]
-        src.append('    } else {')
-        src += ['  ' + s for s in st_cart]
-        src.append('    }')
-        src.append('  }')
-        src.append('}')
-        src.append('')
-        stats = dict(tag=t, cid=cid, L=L, nodes=self.nvar, vrr_flops=self.flops, hrr_flops=self.hrr_flops,
-                     sph_flops=sph_flops, nacc=nacc)
-        return '\n'.join(src), stats
+    # ------------------------------------------------------------ counts
+    def stats(self):
+        """Operation counts of the one-thread schedule: the class's algorithmic work."""
+        self.emit_vrr()
+        self.emit_hrr()
+        self.emit_store(True)
+        return dict(tag=self.tag, cid=class_id(self.la, self.lb, self.lc, self.ld), L=self.L, nodes=self.nvar,
+                    vrr_flops=self.flops, hrr_flops=self.hrr_flops, sph_flops=self.sph_flops,
+                    nacc=len(self.E) * len(self.F))
 
 
 DEFAULT_SLICE_CAP = 8
@@ -410,6 +352,10 @@ def thread_class(c):
     return c[2] + c[3] == 0 or n <= THREAD_TARGETS
 
 
+# ns per quartet with a lane per primitive quartet and with Rys tables (K 1..6,
+# 30 bohr | one primitive on d shells, 8 bohr): 54 targets keep (fs|ds) 18.5 | 11.0
+# against 19.3 | 10.2; above, (pp|pp) with 81 15.2 | 16.4 against 10.1 | 11.1, (dp|ds) with 96
+# 27.5 | 21.9 against 23.6 | 17.2.
 THREAD_TARGETS = 54
 
 # classes on the rotated-axes kernel (warp_emitter.RotationEmitter); ns per
@@ -516,7 +462,7 @@ def emit_all(outdir, lmax=LMAX_EMIT, ngroups=24):
     bodies = []
     for c, fp32 in classes:
         # the one-thread schedule's counts are the algorithmic work of the class
-        st = Emitter(*c).kernel()[1]
+        st = Emitter(*c).stats()
         body, gst = class_source(c, fp32)
         st.update(gst)
         st['fp32'] = fp32
@@ -559,7 +505,7 @@ def emit_all(outdir, lmax=LMAX_EMIT, ngroups=24):
     # uses the class's FP32 kernel (where it measured faster than FP64)
     budget = {b[2]['cid']: b[2]['budget'] for b in bodies}
     minb = [[budget.get(cid) or 0] * 2 + [0] * 2 for cid in range(NCLASS_TOTAL)]
-    # at most 8 lane groups per quartet unless tuned otherwise: measured on the
+    # at most 8 groups per quartet unless tuned otherwise: measured on the
     # screened l <= 2 step (3.4 % of 1e6 quartets kept, primitive screening at
     # 1e-18), a cap of 8 gave 1.18 ms per step against 1.30 uncapped, 1.36 at 2
     # and 1.64 at 1; a class with many quartets runs one group each anyway

@@ -1,4 +1,5 @@
-"""Lane-group ERI kernels: G lanes share one contracted quartet.
+"""Lane-group ERI kernels of the FP32 tier (and the epilogue that the FP64
+kernels of warp_emitter.py share): G lanes share one contracted quartet.
 
 Each lane of a group owns one Cartesian component s of the "lane side" (the bra
 e-range or the ket f-range, whichever has fewer components) and computes, per
@@ -98,17 +99,6 @@ def group_size(n):
 # pack ten-lane groups three to a warp (False: pad them to 16 lanes, two per warp)
 PACK_TEN = True
 
-# lane sides of 21..63 components whose levels below the top fit in fewer than
-# 32 lanes (the S_hi = 4 sides: 20 low + 15 top components): every warp of the
-# group holds all the low levels plus its share of the top level, so the
-# transfer operands stay inside the warp (shuffles, no per-level barrier); the
-# low levels are evaluated once per warp.  Off (False: one copy, transfer
-# operands through shared memory with a named barrier per level): measured on
-# B200, (dd|dd) alone 11.6 ms with it against 10.2 ms without (1e5 quartets,
-# K 1..6), the l <= 2 FP64 step 16.0 against 15.7 ms -- the duplicated chains
-# cost more than the barriers they remove.
-DUP_LOW = False
-
 # register budgets offered to the autotuner: __launch_bounds__(IB_BLOCK, MINB)
 # asks for MINB resident blocks per SM (1: no register cap); must match
 # IB_MINB_VALUES in ib_eri_device.cuh
@@ -136,19 +126,10 @@ class GroupEmitter:
         self.packed = PACK_TEN and self.NL == 10
         if self.packed:
             self.G = 10
-        # duplicated low levels (DUP_LOW): warp q of the group holds every
-        # component below the top level in lanes 0..nlow-1 and top-level
-        # components q*per .. q*per+per-1 in the others
-        self.dup = DUP_LOW and self.NL > 32 and ncum(self.S_hi - 1) < 32
-        if self.dup:
-            self.nlow = ncum(self.S_hi - 1)
-            self.per = 32 - self.nlow
-            self.ntop = ncart(self.S_hi)
-            self.G = 32 * (-(-self.ntop // self.per))
-        # G = 64 or 128: two or four warps per quartet; without dup, transfer
-        # operands go through shared memory, one named barrier per recurrence level
+        # G = 64 or 128: two or four warps per quartet; transfer operands
+        # go through shared memory, one named barrier per recurrence level
         self.wide = self.G > 32
-        self.smem_xfer = self.wide and not self.dup
+        self.smem_xfer = self.wide
         self.QPW = max(1, 32 // self.G)
         self.tag = '%d%d%d%d' % (la, lb, lc, ld)
         self.cid = class_id(la, lb, lc, ld)
@@ -163,12 +144,6 @@ class GroupEmitter:
     def lane_comp(self, j):
         """(component, index of the lane that serves as lane 0 for its transfer
         sources) of group lane j."""
-        if self.dup:
-            w, jw = divmod(j, 32)
-            if jw < self.nlow:
-                return comps_range(0, self.S_hi - 1)[jw], jw
-            t = min(w * self.per + jw - self.nlow, self.ntop - 1)  # padding lanes mirror the last one
-            return comps(self.S_hi)[t], jw
         jj = min(j, self.NL - 1)  # padding lanes mirror the last component
         return comps_range(0, self.S_hi)[jj], jj
 
@@ -250,8 +225,6 @@ class GroupEmitter:
         relative lanes for power-of-two groups, absolute lanes when packed)."""
         if self.packed:
             return '__shfl_sync(gmask, %s, src%d)' % (name, i)
-        if self.dup:
-            return '__shfl_sync(0xffffffffu, %s, src%d, 32)' % (name, i)
         return '__shfl_sync(gmask, %s, src%d, %d)' % (name, i, self.G)
 
     def slot_index(self, c, m):
@@ -645,8 +618,6 @@ class GroupEmitter:
             src.append('  const int gid = threadIdx.x / %d, j = threadIdx.x %% %d;' % (self.G, self.G))
             src.append('  const unsigned gmask = 0xffffffffu;')
             src.append('  const unsigned sgmask = 0xffffffffu;')
-            if self.dup:
-                src.append('  const int jw = j & 31, wq = j >> 5;  // lane in its warp, warp in the group')
         else:
             src.append('  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;')
             src.append('  const int gq = lane / %d, j = lane %% %d;' % (self.G, self.G))
@@ -699,8 +670,6 @@ class GroupEmitter:
         if self.packed:
             src.append('  const int src0 = gq * %d + ((lmisc >> 9) & 127), src1 = gq * %d + ((lmisc >> 16) & 127), '
                        'src2 = gq * %d + ((lmisc >> 23) & 127);' % (self.G, self.G, self.G))
-        elif self.dup:  # lanes of this warp
-            src.append('  const int src0 = (lmisc >> 9) & 31, src1 = (lmisc >> 16) & 31, src2 = (lmisc >> 23) & 31;')
         else:
             src.append('  const int src0 = (lmisc >> 9) & 127, src1 = (lmisc >> 16) & 127, src2 = (lmisc >> 23) & 127;')
         src.append('  const double lcx = (double)(lmisc & 7), lcy = (double)((lmisc >> 3) & 7), '
@@ -710,7 +679,6 @@ class GroupEmitter:
         lane0 = '0' if self.wide else 'lane - r'
         grab = 'ib_grab(a.counter, beg, r, SG, sg, sgmask, %s, lcnt + 2)' % lane0
         src.append('  for (int p = %s; p < end; p = %s) {' % (grab, grab))
-        src.append('    if (sizeof(R) == 8 && a.recheck && !(a.flags[p] & 1)) continue;  // uniform over the quartet\'s lanes')
         src.append('    IbQuartet g;')
         src.append('    ib_load_quartet(a, a.items[p], g);')
         src.append('    const int kb_ = g.k[1], kd_ = g.k[3];')
@@ -719,8 +687,8 @@ class GroupEmitter:
         # side: the screened lists are built here, before the accumulators
         # are live; larger quartets keep exact-zero culling only
         # classes with a g shell build only the exact-zero lists: on the l <= 4
-        # sample workload with primitive screening on, a step of these kernels
-        # (with the low levels then duplicated per warp) stopped on an illegal
+        # sample workload with primitive screening on, a step of an earlier form
+        # of these kernels stopped on an illegal
         # address once; the screened lists stay off for them until that is
         # explained (their exact path ran clean on the same quartets)
         if max(self.la, self.lb, self.lc, self.ld) >= 4:
@@ -754,7 +722,7 @@ class GroupEmitter:
         # FP32 tier: growth of an accumulator's error through the HRRs and
         # transforms; a quartet whose error bound already exceeds the
         # tolerance stops its FP32 primitive loop (the final check rejects it)
-        src.append('    const double famp = sizeof(R) == 4 ? %s : 0.0;' % self.amp_expr())
+        src.append('    const double famp = %s;' % self.amp_expr())
         src.append('    (void)famp;')
         src.append('    for (int ab0 = 0; ab0 < kab; ab0 += 64)')
         src.append('    for (int cd0 = 0; cd0 < kcd; cd0 += 64) {')
@@ -778,14 +746,14 @@ class GroupEmitter:
             src.append('        const int ab = ab0 + lst[qa], cd = cd0 + lst[64 + qc];')
             src.append('        if (ab != ab_last) {')
             src.append('          const int ia = (int)(((float)ab + 0.5f) * rkb), ib = ab - ia * kb_;')
-            src.append('          ib_bra_pair<sizeof(R) == 4>(a, g, ia, ib, bp);')
+            src.append('          ib_bra_pair(a, g, ia, ib, bp);')
             src.append('          ab_last = ab;')
             src.append('        }')
             src.append('        const int ic = (int)(((float)cd + 0.5f) * rkd), id = cd - ic * kd_;')
             src.append('        IbPrimQuartet<R> pq;')
             src.append('        double F[%d];' % (L + 1))
             src.append('        if (!ib_prim_quartet<R, %d>(a, g, bp, ic, id, a.boys_tab, F, pq)) continue;' % L)
-            src.append('        if (sizeof(R) == 4) {')
+            src.append('        {')
             src.append('          est += %s;' % self.err_expr())
             src.append('          if (est * famp > a.mixed_tol) break;  // this slice alone already exceeds it')
             src.append('        }')
@@ -796,15 +764,11 @@ class GroupEmitter:
         else:
             # lane j sets up live primitive quartet q0 + j of the chunk; the
             # group then sweeps the chunk reading the shared values (broadcast)
-            sync = 'ib_group_bar(gid)' if self.smem_xfer else ('__syncwarp()' if self.dup else '__syncwarp(gmask)')
-            # dup: every warp of the group sets up the same chunk of 32
-            # primitive quartets for itself (its own slots of the table)
-            CH = 32 if self.dup else self.G
-            jl = 'jw' if self.dup else 'j'
-            self.chunk = CH
+            sync = 'ib_group_bar(gid)' if self.smem_xfer else '__syncwarp(gmask)'
+            CH = self.G
             src.append('      for (int q0 = w * %d; q0 < npl; q0 += W * %d) {' % (CH, CH))
             src.append('        {')
-            src.append('          const int q = q0 + %s;' % jl)
+            src.append('          const int q = q0 + j;')
             src.append('          if (q < npl) {')
             src.append('            const int qa = (int)(((float)q + 0.5f) * rn1), qc = q - qa * nl1;')
             src.append('            const int ab = ab0 + lst[qa], cd = cd0 + lst[64 + qc];')
@@ -815,7 +779,7 @@ class GroupEmitter:
             src.append('            double F[%d];' % (L + 1))
             src.append('            bool live = !(pre && ib_quartet_negligible(lst, qa, qc, a.prim_tol));')
             src.append('            if (live) {')
-            src.append('              ib_bra_pair<sizeof(R) == 4>(a, g, ia, ib, bp);')
+            src.append('              ib_bra_pair(a, g, ia, ib, bp);')
             src.append('              live = ib_prim_quartet<R, %d>(a, g, bp, ic, id, a.boys_tab, F, pq);' % L)
             src.append('            }')
             src.append('            if (live) {')
@@ -823,17 +787,15 @@ class GroupEmitter:
                 src.append('              ps[%d * %d + j] = pq.%s;' % (k, self.G, f))
             for m in range(L + 1):
                 src.append('              ps[%d * %d + j] = (R)F[%d];' % (len(fields) + m, self.G, m))
-            src.append('              if (sizeof(R) == 4) est += %s;' % self.err_expr())
+            src.append('              est += %s;' % self.err_expr())
             src.append('            }')
             src.append('            pz[j] = live ? 1 : 0;  // 0: pair prefactors multiply to zero, or screened out')
-            # dup: sums of the bound run over this warp's setup lanes only (every
-            # warp of the group set up the same primitive quartets)
             src.append('          }')
             src.append('        }')
             src.append('        %s;' % sync)
             # the group's bound so far (its lanes' partial sums): past the
             # tolerance, the rest of this quartet's FP32 work is skipped
-            src.append('        if (sizeof(R) == 4) {')
+            src.append('        {')
             src.append('          double eg = est;')
             if self.packed:
                 src.append('          sb[%d + j] = est;' % self.red_off)
@@ -841,8 +803,6 @@ class GroupEmitter:
                 src.append('          eg = 0.0;')
                 src.append('          for (int v = 0; v < %d; ++v) eg += sb[%d + v];' % (self.G, self.red_off))
                 src.append('          __syncwarp(gmask);')
-            elif self.dup:
-                src.append('          for (int o = 16; o > 0; o >>= 1) eg += __shfl_xor_sync(0xffffffffu, eg, o);')
             elif self.wide:
                 src.append('          for (int o = 16; o > 0; o >>= 1) eg += __shfl_xor_sync(0xffffffffu, eg, o);')
                 src.append('          if ((j & 31) == 0) sb[%d + (j >> 5)] = eg;' % self.red_off)
@@ -855,13 +815,12 @@ class GroupEmitter:
             src.append('          if (eg * famp > a.mixed_tol) break;  // uniform over the group')
             src.append('        }')
             src.append('        const int nu = min(%d, npl - q0);' % CH)
-            ub = 'wq * 32 + u' if self.dup else 'u'
             src.append('        for (int u = 0; u < nu; ++u) {')
-            src.append('          if (!pz[%s]) continue;  // group-uniform: exact-zero primitive quartet' % ub)
+            src.append('          if (!pz[u]) continue;  // group-uniform: exact-zero primitive quartet')
             for k, nm in enumerate(names):
-                src.append('          const R %s = ps[%d * %d + %s];' % (nm, k, self.G, ub))
+                src.append('          const R %s = ps[%d * %d + u];' % (nm, k, self.G))
             for m in range(L + 1):
-                src.append('        const R f%d = ps[%d * %d + %s];' % (m, len(fields) + m, self.G, ub))
+                src.append('        const R f%d = ps[%d * %d + u];' % (m, len(fields) + m, self.G))
         if bra:
             src.append('        const R SXx = PAx, SXy = PAy, SXz = PAz, SWx = WPx, SWy = WPy, SWz = WPz;')
             src.append('        const R so2 = o2z, sro = roz;')
@@ -901,13 +860,12 @@ class GroupEmitter:
             src.append('      }')
         else:
             src.append('        }')
-            src.append('        %s;' % ('ib_group_bar(gid)' if self.smem_xfer else
-                                        ('__syncwarp()' if self.dup else '__syncwarp(gmask)')))
+            src.append('        %s;' % sync)
             src.append('      }')
         src.append('      ib_sg_sync(SG, sg, sgmask);  // every slice is done with the lists before the next tile')
         src.append('    }')
         # FP32: sum the error bound over the group, reject the quartet if too large
-        src.append('    if (sizeof(R) == 4) {')
+        src.append('    {')
         if self.packed:  # not a power of two: through shared memory
             src.append('      sb[%d + j] = est;' % self.red_off)
             src.append('      __syncwarp(gmask);')
@@ -917,8 +875,6 @@ class GroupEmitter:
         elif self.G > 1 and not self.wide:
             src.append('      for (int o = %d; o > 0; o >>= 1) est += __shfl_xor_sync(gmask, est, o, %d);'
                        % (self.G // 2, self.G))
-        elif self.dup:  # every warp holds the whole group's sum
-            src.append('      for (int o = 16; o > 0; o >>= 1) est += __shfl_xor_sync(0xffffffffu, est, o);')
         elif self.wide:
             src.append('      for (int o = 16; o > 0; o >>= 1) est += __shfl_xor_sync(0xffffffffu, est, o);')
             src.append('      ib_group_bar(gid);')
@@ -940,32 +896,13 @@ class GroupEmitter:
         src.append('      }')
         src.append('    }')
         # accumulators -> shared [e][f]
-        if self.dup:
-            # the row of this lane's component; the low levels are written by
-            # the group's first warp, padding lanes write nothing
-            src.append('    {')
-            src.append('      const int cx = lmisc & 7, cy = (lmisc >> 3) & 7, cz = (lmisc >> 6) & 7, cl = cx + cy + cz;')
-            src.append('      const int crow = cl * (cl + 1) * (cl + 2) / 6 + cz + (cy + cz) * (cy + cz + 1) / 2;')
-            src.append('      const bool mine = jw < %d ? wq == 0 : wq * %d + jw - %d < %d;'
-                       % (self.nlow, self.per, self.nlow, self.ntop))
-            src.append('      if (mine && crow >= %d) {' % s_lo_idx)
-            for tt in range(NT):
-                if bra:
-                    src.append('        sb[(crow - %d) * %d + %d] = acc[%d];' % (s_lo_idx, NFP, tt, tt))
-                else:
-                    src.append('        sb[%d * %d + (crow - %d)] = acc[%d];' % (tt, NFP, s_lo_idx, tt))
-            src.append('      }')
-            src.append('    }')
-        else:
+        src.append('    if (j >= %d && j < %d) {' % (s_lo_idx, self.NL))
+        for tt in range(NT):
             if bra:
-                src.append('    if (j >= %d && j < %d) {' % (s_lo_idx, self.NL))
-                for tt in range(NT):
-                    src.append('      sb[(j - %d) * %d + %d] = acc[%d];' % (s_lo_idx, NFP, tt, tt))
+                src.append('      sb[(j - %d) * %d + %d] = acc[%d];' % (s_lo_idx, NFP, tt, tt))
             else:
-                src.append('    if (j >= %d && j < %d) {' % (s_lo_idx, self.NL))
-                for tt in range(NT):
-                    src.append('      sb[%d * %d + (j - %d)] = acc[%d];' % (tt, NFP, s_lo_idx, tt))
-            src.append('    }')
+                src.append('      sb[%d * %d + (j - %d)] = acc[%d];' % (tt, NFP, s_lo_idx, tt))
+        src.append('    }')
         src.append('    ib_sg_sync(SG, sg, sgmask);')
         src.append('    if (W > 1) {  // slice 0 table += the other slices tables')
         src.append('      for (int x = r; x < %d; x += SG) {' % (NE * NF))

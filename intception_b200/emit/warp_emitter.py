@@ -26,6 +26,19 @@ lane evaluates a value twice, and nothing is exchanged between dependent
 recurrence levels.  Several primitive quartets share a warp in the product step
 (QPW = 32 // targets); lane sides of more than 32 targets take several warps, and
 chain sides of more than MAX_ACC targets are split over warps as well.
+
+What bounds them (B200, FP64): the large classes' product step, its shared loads
+(69-76 % of the load/store unit's cycles on (dp|dp) and (dd|dd); every lane reads
+its own 3 (C + 1) integrals of a root, so a wider chain side is read less often
+per product: plan() weighs the two), the classes with few primitive quartets
+latency at 12-16 warps an SM.  ns per quartet, K 1..6 in a 30-bohr box, against
+the lane-group kernels of the recurrences (group_emitter.py) that these replace:
+(ss|ss) 8.1 -> 2.9, (ps|ps) 10.5 -> 3.7, (pp|ps) 12.5 -> 5.1, (dp|dp) 55 -> 28,
+(dd|dd) 110 -> 56, (fd|dd) 297 -> 170, (ff|dd) 1082 -> 785; (ff|ff) is level (1.9 us).
+With few primitives (s shells of 3 or 6, p of 3, d and f of one, 8 bohr):
+(ss|ss) 12.7 -> 4.1, (dd|dd) 16.1 -> 8.5, (ff|dd) 48 -> 33, but (ds|ds) 4.1 -> 5.2 and
+(dd|ds) 6.3 -> 7.6: ten-lane groups put three such quartets in a warp, a warp
+here holds one.
 """
 from intception_b200.basis import sph_matrix
 
@@ -593,7 +606,9 @@ class ThreadEmitter(WarpEmitter):
     """Kernel whose lanes take a primitive quartet each and run the whole
     Obara-Saika recurrence for all targets in registers (the one-thread schedule
     of eri_emitter.Emitter); the lanes' sums meet in shared memory.  For classes
-    whose [e0|f0] table is small enough to be a lane's accumulators."""
+    whose [e0|f0] table is small enough to be a lane's accumulators.  Bound by
+    the FP64 pipe and the Boys table gathers where K is large, by latency where
+    a quartet has fewer primitive quartets than lanes."""
 
     kind = 'thread'
     PASS = 32  # accumulators per reduction pass
@@ -686,7 +701,8 @@ class RotationEmitter(WarpEmitter):
     fall into orbits of the cyclic axis permutation (x, xx, xy stand for all
     nine of levels 1 and 2), so lane k evaluates one representative of each
     with its axes rotated by k: the same instructions on every lane, every 2D
-    integral in the lane's registers, no step between roots and products."""
+    integral in the lane's registers, no step between roots and products.  Bound
+    by the FP64 pipe and its latency; figures at eri_emitter.ROTATED."""
 
     kind = 'rot'
     ORBITS = {(1, 0): ((1, 0, 0),), (1, 1): ((1, 0, 0), (2, 0, 0), (1, 1, 0)), (2, 0): ((2, 0, 0), (1, 1, 0))}
