@@ -30,13 +30,27 @@ __device__ __forceinline__ void jk_comp(int l, int k, int& x, int& y, int& z) {
   x = l - s;
 }
 
+// y + z of component k
+__device__ __forceinline__ int jk_yz(int k) {
+  return (k >= 1) + (k >= 3) + (k >= 6) + (k >= 10) + (k >= 15) + (k >= 21);
+}
+
 __device__ __forceinline__ int jk_index(int x, int y, int z) { return z + (y + z) * (y + z + 1) / 2; }
 
+// The six density values of an element (P is symmetric).  A warp's elements run
+// through i, then j, and few k and l: rows k and l put their values into one line
+// each, where rows i and j would take a line a value.
+struct JkP {
+  double ij, kl, ki, lj, li, kj;
+};
+__device__ __forceinline__ JkP jk_density(const double* __restrict__ P, int n, int i, int j, int k, int l) {
+  const double* __restrict__ Pk = P + (size_t)k * n;
+  const double* __restrict__ Pl = P + (size_t)l * n;
+  return {__ldg(P + (size_t)i * n + j), __ldg(Pk + l), __ldg(Pk + i), __ldg(Pl + j), __ldg(Pl + i), __ldg(Pk + j)};
+}
 __device__ __forceinline__ double jk_weight(const double* __restrict__ P, int n, int i, int j, int k, int l) {
-  const double pij = __ldg(P + (size_t)i * n + j), pkl = __ldg(P + (size_t)k * n + l);
-  const double pik = __ldg(P + (size_t)i * n + k), pjl = __ldg(P + (size_t)j * n + l);
-  const double pil = __ldg(P + (size_t)i * n + l), pjk = __ldg(P + (size_t)j * n + k);
-  return 0.5 * pij * pkl - 0.125 * (pik * pjl + pil * pjk);
+  const JkP p = jk_density(P, n, i, j, k, l);
+  return 0.5 * p.ij * p.kl - 0.125 * (p.ki * p.lj + p.li * p.kj);
 }
 
 __device__ __forceinline__ double jk_deg(const int* s) {
@@ -70,11 +84,17 @@ __device__ __forceinline__ JkDD jk_dd_add(JkDD a, JkDD b) {
   return r;
 }
 
+// e / n for the element indices of a block (e < 28^4 < 2^21, n <= 28): (e + 0.5) / n
+// is at least 0.5 / n away from an integer, the two roundings are below that.
+__device__ __forceinline__ int jk_quot(int e, float rn) { return (int)(((float)e + 0.5f) * rn); }
+
 // One warp per quartet.  Each lane sums its shares in plain double (a few
 // hundred terms, a fixed order), the warp, block and grid sums are
 // double-double: block k writes its (E_J, E_K) partials to part[4k .. 4k+3]
 // and ib_jk_energy_finish adds them in block order into e_out.  The result
-// does not depend on scheduling.
+// does not depend on scheduling.  27 atoms, l <= 2: 5.75 ms an energy, 6.22 with
+// integer divisions and densities read along the rows of i and j, 6.24 with
+// two quartets a warp (neighbours in the list differ in size).
 __global__ void ib_jk_energy_kernel(const int* __restrict__ quartets, const long long* __restrict__ out_off, int nq,
                                     const int* __restrict__ shell_l, const int* __restrict__ fofs,
                                     const double* __restrict__ P, int nbf, const double* __restrict__ blocks,
@@ -85,24 +105,24 @@ __global__ void ib_jk_energy_kernel(const int* __restrict__ quartets, const long
   double sj = 0.0, sk = 0.0;  // this lane's plain sums: a few hundred terms in a fixed order
   for (int q = warp; q < nq; q += nwarp) {
     int s[4], n[4], f[4];
+#pragma unroll
     for (int i = 0; i < 4; ++i) {
-      s[i] = quartets[4 * q + i];
-      n[i] = ib_ncart(shell_l[s[i]]);
-      f[i] = fofs[s[i]];
+      s[i] = __ldg(quartets + 4 * (size_t)q + i);
+      n[i] = ib_ncart(__ldg(shell_l + s[i]));
+      f[i] = __ldg(fofs + s[i]);
     }
     const double deg = jk_deg(s);
-    const double* blk = blocks + out_off[q];
+    const double* __restrict__ blk = blocks + __ldg(out_off + q);
     const int tot = n[0] * n[1] * n[2] * n[3];
+    const float rn0 = 1.0f / (float)n[0], rn1 = 1.0f / (float)n[1], rn2 = 1.0f / (float)n[2];
     double pj = 0.0, pk = 0.0;
     for (int e = lane; e < tot; e += 32) {
-      const int ia = e % n[0], r1 = e / n[0];
-      const int ib = r1 % n[1], r2 = r1 / n[1];
-      const int ic = r2 % n[2], id = r2 / n[2];
-      const int i = f[0] + ia, j = f[1] + ib, k = f[2] + ic, l = f[3] + id;
-      const double v = blk[e];
-      pj += __ldg(P + (size_t)i * nbf + j) * __ldg(P + (size_t)k * nbf + l) * v;
-      pk += (__ldg(P + (size_t)i * nbf + k) * __ldg(P + (size_t)j * nbf + l) +
-             __ldg(P + (size_t)i * nbf + l) * __ldg(P + (size_t)j * nbf + k)) * v;
+      const int r1 = jk_quot(e, rn0), r2 = jk_quot(r1, rn1), id = jk_quot(r2, rn2);
+      const int i = f[0] + e - r1 * n[0], j = f[1] + r1 - r2 * n[1], k = f[2] + r2 - id * n[2], l = f[3] + id;
+      const JkP p = jk_density(P, nbf, i, j, k, l);
+      const double v = __ldg(blk + e);
+      pj += p.ij * p.kl * v;
+      pk += (p.ki * p.lj + p.li * p.kj) * v;
     }
     sj += 0.5 * deg * pj;
     sk -= 0.125 * deg * pk;
@@ -277,6 +297,14 @@ __global__ void ib_jk_force_kernel(const int* __restrict__ quartets, const int* 
 // for each centre pos and direction x
 //   dE/dA_pos,x += deg W(o) [(o + 1x | raised at pos) - o_x (o - 1x | lowered at pos)],
 // the adjoint of the derivative rule above; centre D takes the opposite sum.
+//
+// 20 atoms, l <= 2 (screen 1e-15): 14.6 ms of a gradient before, 10.8 now, by
+// quotients in float instead of integer divisions, 16 exchanges a quartet
+// instead of 45, one shared add a lane instead of 18 in turn, and densities read
+// along the rows of k and l.  Staging the six density blocks in shared memory
+// (ib_jk_force_kernel's way) made it 12.4: its 38 KB a block cost more
+// occupancy than the gathers cost time.  Fetching the next quartet's indices
+// early changed nothing (11.1).
 struct JkAux {
   const long long* off[6];
   const double* blk[6];
@@ -287,94 +315,80 @@ __global__ void ib_jk_force_all_kernel(const int* __restrict__ quartets, int nq,
                                        const int* __restrict__ shell_atom, const double* __restrict__ P, int nbf,
                                        int natom, double* __restrict__ force) {
   extern __shared__ double fs[];
-  double* stage = fs + ((3 * natom + 1) & ~1);
   for (int i = threadIdx.x; i < 3 * natom; i += blockDim.x) fs[i] = 0.0;
   __syncthreads();
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double* __restrict__ st = stage + (size_t)wib * 6 * JK_STAGE_N * JK_STAGE_N;
-  const int SS = JK_STAGE_N * JK_STAGE_N;
+  const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarp = (gridDim.x * blockDim.x) >> 5;
   for (int q = warp; q < nq; q += nwarp) {
     int s[4], l[4], n[4], f[4];
+    long long off[6];
+#pragma unroll
     for (int i = 0; i < 4; ++i) {
-      s[i] = quartets[4 * q + i];
-      l[i] = shell_l[s[i]];
-      f[i] = fofs[s[i]];
+      s[i] = __ldg(quartets + 4 * (size_t)q + i);
+      l[i] = __ldg(shell_l + s[i]);
+      f[i] = __ldg(fofs + s[i]);
       n[i] = ib_ncart(l[i]);
     }
-    long long off[6];
+#pragma unroll
     for (int b = 0; b < 6; ++b) off[b] = __ldg(aux.off[b] + q);
     const double deg = jk_deg(s);
     const int tot = n[0] * n[1] * n[2] * n[3];
-    const bool staged = max(max(l[0], l[1]), max(l[2], l[3])) <= JK_STAGE_L && tot >= 128;
-    if (staged) {
-      __syncwarp();
-      jk_stage(P, nbf, f[0], n[0], f[1], n[1], st + 0 * SS, lane);
-      jk_stage(P, nbf, f[2], n[2], f[3], n[3], st + 1 * SS, lane);
-      jk_stage(P, nbf, f[0], n[0], f[2], n[2], st + 2 * SS, lane);
-      jk_stage(P, nbf, f[1], n[1], f[3], n[3], st + 3 * SS, lane);
-      jk_stage(P, nbf, f[0], n[0], f[3], n[3], st + 4 * SS, lane);
-      jk_stage(P, nbf, f[1], n[1], f[2], n[2], st + 5 * SS, lane);
-      __syncwarp();
-    }
-    double g[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // [pos][x]
+    const float rn[3] = {1.0f / (float)n[0], 1.0f / (float)n[1], 1.0f / (float)n[2]};
+    double g[16];  // [pos][x], zeros up to a power of two
+#pragma unroll
+    for (int k = 0; k < 16; ++k) g[k] = 0.0;
     for (int e = lane; e < tot; e += 32) {
-      int idx[4];
-      int r = e;
-      for (int i = 0; i < 4; ++i) {
-        idx[i] = r % n[i];
-        r /= n[i];
+      int r[4], idx[4];  // r[i]: index over shells i and later
+      r[0] = e;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        r[i + 1] = jk_quot(r[i], rn[i]);
+        idx[i] = r[i] - r[i + 1] * n[i];
       }
-      double w;
-      if (staged) {
-        const int N = JK_STAGE_N;
-        w = 0.5 * st[0 * SS + idx[0] * N + idx[1]] * st[1 * SS + idx[2] * N + idx[3]] -
-            0.125 * (st[2 * SS + idx[0] * N + idx[2]] * st[3 * SS + idx[1] * N + idx[3]] +
-                     st[4 * SS + idx[0] * N + idx[3]] * st[5 * SS + idx[1] * N + idx[2]]);
-      } else {
-        w = jk_weight(P, nbf, f[0] + idx[0], f[1] + idx[1], f[2] + idx[2], f[3] + idx[3]);
-      }
-      w *= deg;
+      idx[3] = r[3];
+      const double w = deg * jk_weight(P, nbf, f[0] + idx[0], f[1] + idx[1], f[2] + idx[2], f[3] + idx[3]);
+      int stride = 1;
+#pragma unroll
       for (int pos = 0; pos < 3; ++pos) {
-        int cx, cy, cz;
-        jk_comp(l[pos], idx[pos], cx, cy, cz);
-        const int c[3] = {cx, cy, cz};
-        // flat index of the block with component k at pos and extent m there
-        int lo = 0, stride = 1;  // contribution of the indices before pos, stride of pos
-        for (int i = 0; i < pos; ++i) {
-          lo += idx[i] * stride;
-          stride *= n[i];
+        // component k = t (t + 1) / 2 + z of x = l - t, y + z = t: one more x keeps
+        // the index, one more y adds t + 1, one more z adds t + 2
+        const int k = idx[pos], t = jk_yz(k), z = k - t * (t + 1) / 2;
+        const int lo = e - stride * r[pos];
+        const double* bp = aux.blk[2 * pos] + off[2 * pos] + lo + stride * (k + ib_ncart(l[pos] + 1) * r[pos + 1]);
+        double v[3] = {__ldg(bp), __ldg(bp + stride * (t + 1)), __ldg(bp + stride * (t + 2))};
+        if (off[2 * pos + 1] >= 0) {
+          const double* bm =
+              aux.blk[2 * pos + 1] + off[2 * pos + 1] + lo + stride * (k + ib_ncart(l[pos] - 1) * r[pos + 1]);
+          if (l[pos] > t) v[0] -= (double)(l[pos] - t) * __ldg(bm);
+          if (t > z) v[1] -= (double)(t - z) * __ldg(bm - stride * t);
+          if (z > 0) v[2] -= (double)z * __ldg(bm - stride * (t + 1));
         }
-        int hi = 0, hs = 1;  // indices after pos, in units of the stride after pos
-        for (int i = pos + 1; i < 4; ++i) {
-          hi += idx[i] * hs;
-          hs *= n[i];
-        }
-        const int np1 = ib_ncart(l[pos] + 1), nm1 = ib_ncart(l[pos] - 1);
-        const double* bp = aux.blk[2 * pos] + off[2 * pos];
-        const double* bm = off[2 * pos + 1] >= 0 ? aux.blk[2 * pos + 1] + off[2 * pos + 1] : nullptr;
-        for (int x = 0; x < 3; ++x) {
-          int o[3] = {c[0], c[1], c[2]};
-          o[x] += 1;
-          double v = __ldg(bp + lo + stride * (jk_index(o[0], o[1], o[2]) + np1 * hi));
-          if (c[x] > 0 && bm) {
-            o[x] -= 2;
-            v -= (double)c[x] * __ldg(bm + lo + stride * (jk_index(o[0], o[1], o[2]) + nm1 * hi));
-          }
-          g[3 * pos + x] += w * v;
-        }
+#pragma unroll
+        for (int x = 0; x < 3; ++x) g[3 * pos + x] += w * v[x];
+        stride *= n[pos];
       }
     }
-    for (int k = 0; k < 9; ++k) g[k] = warp_sum(g[k]);
-    if (lane == 0) {
-      const int ad = shell_atom[s[3]];
-      for (int pos = 0; pos < 3; ++pos) {
-        const int ax = shell_atom[s[pos]];
-        for (int x = 0; x < 3; ++x) {
-          atomicAdd(&fs[3 * ax + x], g[3 * pos + x]);
-          atomicAdd(&fs[3 * ad + x], -g[3 * pos + x]);
-        }
+    // sums over the lanes: each step halves the values that a lane holds, so
+    // that lanes 2k and 2k + 1 end with the sum of value k (16 exchanges, not 45)
+#pragma unroll
+    for (int o = 16, m = 8; m > 0; o >>= 1, m >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int k = 0; k < m; ++k) {
+        const double give = up ? g[k] : g[k + m], keep = up ? g[k + m] : g[k];
+        g[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
       }
+    }
+    const double sum = g[0] + __shfl_xor_sync(0xffffffffu, g[0], 1);
+    // even lanes add a value to its centre; odd lanes 1, 3, 5 the opposite of a
+    // direction's three to centre D (one lane after the other took 18 adds in turn)
+    const int k = lane >> 1, x = k % 3;
+    const double dx = __shfl_sync(0xffffffffu, sum, 2 * x) + __shfl_sync(0xffffffffu, sum, 2 * x + 6) +
+                      __shfl_sync(0xffffffffu, sum, 2 * x + 12);
+    const bool centre_d = lane & 1;
+    if (k < (centre_d ? 3 : 9)) {
+      const int at = centre_d ? s[3] : k < 3 ? s[0] : k < 6 ? s[1] : s[2];
+      atomicAdd(&fs[3 * shell_atom[at] + x], centre_d ? -dx : sum);
     }
   }
   __syncthreads();
@@ -445,8 +459,7 @@ extern "C" int intception_b200_jk_force_all(const int* quartets, int nq, const l
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return IB_ERR_NODEVICE;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem =
-      sizeof(double) * (((3 * (size_t)natom + 1) & ~(size_t)1) + (size_t)JK_WARPS * 6 * JK_STAGE_N * JK_STAGE_N);
+  const size_t smem = sizeof(double) * 3 * (size_t)natom;
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(ib_jk_force_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess)
