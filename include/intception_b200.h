@@ -173,7 +173,10 @@ int intception_b200_eri_batch(const intception_b200_basis *basis, const int *qua
  * launch.  create runs the batch once eagerly (sizing the work buffers, so the
  * capture allocates nothing) and once under capture; launch replays it on
  * stream; replays read the inputs' current contents.  The graph uses the
- * library's shared work buffers: do not run it concurrently with other batches. */
+ * library's shared work buffers: do not run it concurrently with other batches.
+ * Batches of any size may run between replays: a work buffer that the library
+ * outgrows stays allocated until the last graph is destroyed (for good when a
+ * caller captured eri_batch on a stream of its own). */
 int intception_b200_eri_graph_create(const intception_b200_basis *basis, const int *quartets,
                                      const long long *out_off, int nq, int spherical, int precision,
                                      const double *bounds, double skip_below, double fp32_below, double mixed_tol,

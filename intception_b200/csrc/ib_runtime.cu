@@ -97,9 +97,15 @@ int pair_index_h(int la, int lb) { return la * (la + 1) / 2 + lb; }
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
-  cudaError_t ensure(size_t bytes) {
+  bool captured = false;  // a captured batch holds this block's address
+  // kept: where an outgrown captured block goes instead of being freed
+  cudaError_t ensure(size_t bytes, std::vector<void*>* kept = nullptr) {
     if (bytes <= cap) return cudaSuccess;
-    if (p) cudaFree(p);
+    if (p && captured && kept)
+      kept->push_back(p);
+    else if (p)
+      cudaFree(p);
+    captured = false;
     p = nullptr;
     cap = 0;
     size_t want = std::max(bytes, cap + cap / 2);
@@ -159,7 +165,8 @@ struct Context {
   int* status = nullptr;  // status word of every batch, whichever path it takes (the first control word)
   const int* last_status = nullptr;  // status word and redo list of the last batch
   const int* last_redo = nullptr;    // (null after a drop-in call: the host copies)
-  int host_status = 0, host_redo = 0;
+  const int* last_flags = nullptr;   // its FP32 rejection flags (flags_nq of them)
+  int host_status = 0, host_redo = 0, host_rejections = 0;
   DevBuf redo;     // the last batch's redo lists (redo_groups of them, redo_stride ints apart; IbLaunch::redo)
   int redo_groups = 1, redo_stride = 2;
   DevBuf tickets;  // kTickets ints: the generic kernel's ticket pairs (zeroed by every dispatch)
@@ -168,6 +175,54 @@ struct Context {
   int kind_h[IB_NCLASS] = {};  // host copy of kind: 2 where the class has FP32 kernels and the FP32 tier uses them
   DevBuf d_stage, d_cart, d_res;
   HostBuf h_stage, h_res;
+  // Work buffers that a captured batch replays with: an outgrown block stays
+  // allocated while a graph may still use it (kept), one set per captured size
+  // at most.  A batch captured on the caller's own stream (not by
+  // eri_graph_create) keeps its blocks for good: its end is not known here.
+  std::vector<void*> kept;
+  int graphs = 0;                // graphs of eri_graph_create alive
+  bool foreign_capture = false;  // a batch was captured on the caller's stream
+  void mark_captured(bool on) {
+    for (DevBuf* b : {&keys, &vals, &keys2, &vals2, &items, &cub_tmp, &scratch, &flags, &redo}) b->captured = on;
+  }
+  void release_kept() {  // with the last graph
+    if (graphs > 0 || foreign_capture) return;
+    // counts of a last batch whose lists lie in a kept block move to the host
+    if (std::count(kept.begin(), kept.end(), (void*)last_redo)) {
+      read_redo(&host_redo);
+      last_redo = nullptr;
+    }
+    if (std::count(kept.begin(), kept.end(), (void*)last_flags)) {
+      read_rejections(&host_rejections);
+      last_flags = nullptr;
+    }
+    for (void* q : kept) cudaFree(q);  // waits for replays still in flight
+    kept.clear();
+    mark_captured(false);
+  }
+  // Redo list entries and FP32 rejections of the last batch (synchronous).
+  cudaError_t read_redo(int* total) const {
+    *total = host_redo;
+    if (!last_redo) return cudaSuccess;
+    cudaError_t e = cudaDeviceSynchronize();
+    *total = 0;
+    for (int g = 0; g < redo_groups && e == cudaSuccess; ++g) {
+      int h[2] = {0, 0};  // heavy and light counts
+      e = cudaMemcpy(h, last_redo + (size_t)g * redo_stride, 2 * sizeof(int), cudaMemcpyDeviceToHost);
+      *total += h[0] + h[1];
+    }
+    return e;
+  }
+  cudaError_t read_rejections(int* total) const {
+    *total = host_rejections;
+    if (!last_flags) return cudaSuccess;
+    cudaError_t e = cudaDeviceSynchronize();
+    // only the last batch's flags: the buffer keeps stale entries past them
+    std::vector<int> h(flags_nq);
+    if (e == cudaSuccess) e = cudaMemcpy(h.data(), last_flags, h.size() * sizeof(int), cudaMemcpyDeviceToHost);
+    *total = (int)std::count_if(h.begin(), h.end(), [](int v) { return v & 1; });
+    return e;
+  }
   IbClassEntry table[IB_NCLASS] = {};
   int occ[IB_NCLASS][4 * IB_NMINB] = {};
   int minb_idx[IB_NCLASS][4] = {};  // register budget chosen per class and variant (autotuned defaults)
@@ -642,7 +697,7 @@ cudaError_t redo_launch(Context* c, cudaStream_t s, const IbLaunch& a, bool sph,
   long long nblk = std::min<long long>((long long)ib_generic_bps() * c->nsm,
                                       (long long)(kScratchCap / (slice * sizeof(double))));
   nblk = std::max<long long>(nblk, 1);
-  cudaError_t e = c->scratch.ensure((size_t)nblk * slice * sizeof(double));
+  cudaError_t e = c->scratch.ensure((size_t)nblk * slice * sizeof(double), &c->kept);
   if (e != cudaSuccess) return e;
   const IbGenWork wk{-1, 0, 1, tickets, ib_generic_split() >= 1 ? kSplitRedo : 0};
   return ib_generic_launch((int)nblk, s, a, wk, sph ? 1 : 0, c->scratch.as<double>(), slice);
@@ -702,7 +757,7 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, int nq, bool fp64_pr
   const long long gfull = std::max<long long>(
       1, std::min<long long>((long long)ib_generic_bps() * c->nsm, (long long)(kScratchCap / (gslice * sizeof(double)))));
   const long long ggroup = gfull;  // each group's redo may take the whole GPU once the others are done
-  if (G > 1) IB_CUDA(c->scratch.ensure((size_t)(gfull + G * ggroup) * gslice * sizeof(double)));
+  if (G > 1) IB_CUDA(c->scratch.ensure((size_t)(gfull + G * ggroup) * gslice * sizeof(double), &c->kept));
   // screened quartets: zero blocks, concurrent with the class kernels (launched
   // first with 4 blocks per SM: measured no slower than 1 or 2 blocks per SM, or
   // than launching it after the class kernels)
@@ -716,7 +771,7 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, int nq, bool fp64_pr
   // empty range returns at once).  From lmax 3 its range is the longest job
   // of a batch, so it starts first; below, after the class kernels.
   auto launch_generic = [&]() -> cudaError_t {
-    cudaError_t e = c->scratch.ensure((size_t)(gfull + (G > 1 ? G * ggroup : 0)) * gslice * sizeof(double));
+    cudaError_t e = c->scratch.ensure((size_t)(gfull + (G > 1 ? G * ggroup : 0)) * gslice * sizeof(double), &c->kept);
     if (e != cudaSuccess) return e;
     // heavy quartets of the range over clusters too (INTCEPTION_B200_GENERIC_SPLIT 2)
     e = ib_generic_launch((int)gfull, c->side[k % nuse], a,
@@ -974,9 +1029,8 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
   a.prim_coef = reinterpret_cast<const double*>(d + o_c);
   a.out = sph ? c->d_cart.as<double>() : dres;
   a.status = reinterpret_cast<int*>(d + o_status);
-  c->last_status = c->last_redo = nullptr;  // read from the host copies below
-  c->host_status = c->host_redo = 0;
-  c->flags_nq = 0;
+  c->last_status = c->last_redo = c->last_flags = nullptr;  // read from the host copies below
+  c->host_status = c->host_redo = c->host_rejections = 0;
   if (emitted) {
     const int vt = 4 * c->minb_idx[cidx][0];
     const int grid = std::max(1, std::min(c->nsm * c->occ[cidx][vt], nblk));
@@ -991,7 +1045,7 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
     long long nb = std::min<long long>({(long long)nblk, (long long)ib_generic_bps() * c->nsm,
                                         (long long)(kScratchCap / (slice * sizeof(double)))});
     nb = std::max<long long>(nb, 1);
-    IB_CUDA(c->scratch.ensure((size_t)nb * slice * sizeof(double)));
+    IB_CUDA(c->scratch.ensure((size_t)nb * slice * sizeof(double), &c->kept));
     IB_CUDA(ib_generic_launch((int)nb, s, a, IbGenWork{-1, kSlotGenLight, 0, nullptr}, 0, c->scratch.as<double>(),
                               slice));
   }
@@ -1179,7 +1233,8 @@ int small_batch(Context* c, const intception_b200_basis* basis, const int* quart
   c->last_status = ctl;
   c->last_redo = a.redo;
   c->redo_groups = 1;
-  c->flags_nq = 0;
+  c->last_flags = nullptr;
+  c->flags_nq = c->host_rejections = 0;
   const IbSmallArgs b = {quartets, out_off, bounds, skip_below, c->small_items.as<IbItem>(), nq, basis->lmax};
   const int grid = std::min(2 * c->nsm, nq);
   IB_CUDA(spherical ? ib_small_launch_sph(grid, s, a, b) : ib_small_launch_cart(grid, s, a, b));
@@ -1207,20 +1262,23 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   if (nq <= kSmallBatch && basis->lmax <= ib_lmax_emitted && precision == IB_PREC_FP64 && c->hrr_tol > 0.0)
     return small_batch(c, basis, quartets, out_off, nq, spherical, skip_below > 0.0 ? bounds : nullptr, skip_below, out,
                        s, nl, screen_prims);
-  IB_CUDA(c->keys.ensure((size_t)nq * sizeof(unsigned)));
-  IB_CUDA(c->keys2.ensure((size_t)nq * sizeof(unsigned)));
-  IB_CUDA(c->vals.ensure((size_t)nq * sizeof(int)));
-  IB_CUDA(c->vals2.ensure((size_t)nq * sizeof(int)));
-  IB_CUDA(c->items.ensure((size_t)nq * sizeof(IbItem)));
+  c->last_redo = c->last_flags = nullptr;  // their blocks may move
+  c->host_redo = c->host_rejections = 0;
+  IB_CUDA(c->keys.ensure((size_t)nq * sizeof(unsigned), &c->kept));
+  IB_CUDA(c->keys2.ensure((size_t)nq * sizeof(unsigned), &c->kept));
+  IB_CUDA(c->vals.ensure((size_t)nq * sizeof(int), &c->kept));
+  IB_CUDA(c->vals2.ensure((size_t)nq * sizeof(int), &c->kept));
+  IB_CUDA(c->items.ensure((size_t)nq * sizeof(IbItem), &c->kept));
   size_t tmp_bytes = 0;
   IB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, c->keys.as<unsigned>(), c->keys2.as<unsigned>(),
                                           c->vals.as<int>(), c->vals2.as<int>(), nq, 0, kKeyBits, s));
-  IB_CUDA(c->cub_tmp.ensure(tmp_bytes));
-  IB_CUDA(c->flags.ensure((size_t)nq * sizeof(int)));
+  IB_CUDA(c->cub_tmp.ensure(tmp_bytes, &c->kept));
+  IB_CUDA(c->flags.ensure((size_t)nq * sizeof(int), &c->kept));
   // l >= 3 batches: four redo lists, one per group of side streams (dispatch)
   c->redo_groups = (basis->lmax >= 3 && c->hrr_tol > 0.0) ? kRedoGroups : 1;
   c->redo_stride = nq + 2;
-  IB_CUDA(c->redo.ensure((size_t)c->redo_groups * (nq + 2) * sizeof(int)));
+  IB_CUDA(c->redo.ensure((size_t)c->redo_groups * (nq + 2) * sizeof(int), &c->kept));
+  c->last_flags = c->flags.as<int>();
   c->flags_nq = nq;
   c->last_status = c->status;
   c->last_redo = c->redo.as<int>();
@@ -1396,6 +1454,12 @@ int intception_b200_eri_batch(const intception_b200_basis* basis, const int* qua
   int nl = 0;
   st = batch_impl(c, basis, quartets, out_off, nq, spherical, precision, bounds, skip_below, fp32_below, mixed_tol,
                   out, s, &nl);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) (void)cudaGetLastError();  // (the launches report it)
+  if (cap == cudaStreamCaptureStatusActive) {
+    c->foreign_capture = true;
+    c->mark_captured(true);
+  }
   tl_launches = nl;
   if (st) return st;
   return set_status(IB_OK, "");
@@ -1481,8 +1545,9 @@ struct IbGraph {
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   int launches;
-  int nq;
-  bool small;  // captured the small-batch kernel: its redo list lies in the control words
+  // what the status and redo queries read after a replay: the captured blocks,
+  // which the context may have outgrown since
+  const int *redo, *flags;
   int flags_nq, redo_groups, redo_stride;
 };
 
@@ -1506,7 +1571,7 @@ int intception_b200_eri_graph_create(const intception_b200_basis* basis, const i
     return st;
   }
   IB_CUDA(cudaStreamSynchronize(s));
-  IbGraph* g = new IbGraph{c, nullptr, nullptr, 0, nq, c->last_redo != c->redo.as<int>(), c->flags_nq, c->redo_groups,
+  IbGraph* g = new IbGraph{c, nullptr, nullptr, 0, c->last_redo, c->last_flags, c->flags_nq, c->redo_groups,
                            c->redo_stride};
   IB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   nl = 0;
@@ -1528,6 +1593,8 @@ int intception_b200_eri_graph_create(const intception_b200_basis* basis, const i
     delete g;
     return set_status(IB_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ei));
   }
+  ++c->graphs;
+  c->mark_captured(true);
   *handle = g;
   return set_status(IB_OK, "");
 }
@@ -1540,7 +1607,8 @@ int intception_b200_eri_graph_launch(void* handle, void* stream) {
   Context* c = g->ctx;
   std::lock_guard<std::mutex> lk(c->mu);
   c->last_status = c->status;
-  c->last_redo = g->small ? c->status + 16 + g->nq : c->redo.as<int>();
+  c->last_redo = g->redo;
+  c->last_flags = g->flags;
   c->flags_nq = g->flags_nq;
   c->redo_groups = g->redo_groups;
   c->redo_stride = g->redo_stride;
@@ -1551,9 +1619,13 @@ int intception_b200_eri_graph_launch(void* handle, void* stream) {
 int intception_b200_eri_graph_destroy(void* handle) {
   IbGraph* g = static_cast<IbGraph*>(handle);
   if (!g) return set_status(IB_OK, "");
+  Context* c = g->ctx;
+  std::lock_guard<std::mutex> lk(c->mu);
   cudaGraphExecDestroy(g->exec);
   cudaGraphDestroy(g->graph);
   delete g;
+  --c->graphs;
+  c->release_kept();
   return set_status(IB_OK, "");
 }
 
@@ -1562,15 +1634,10 @@ int intception_b200_eri_graph_destroy(void* handle) {
 int intception_b200_last_fp32_rejections(void) {
   Context* c = nullptr;
   if (get_context(&c)) return -1;
-  if (!c->flags.p || c->flags_nq <= 0) return 0;
-  IB_CUDA(cudaDeviceSynchronize());
-  // only the last batch's flags: the buffer keeps stale entries past them
-  const size_t n = std::min((size_t)c->flags_nq, c->flags.cap / sizeof(int));
-  std::vector<int> h(n);
-  IB_CUDA(cudaMemcpy(h.data(), c->flags.p, n * sizeof(int), cudaMemcpyDeviceToHost));
-  int k = 0;
-  for (int v : h) k += v & 1;
-  return k;
+  std::lock_guard<std::mutex> lk(c->mu);
+  int total = 0;
+  IB_CUDA(c->read_rejections(&total));
+  return total;
 }
 
 // Number of quartets of the last batch (or drop-in call) that the class
@@ -1579,14 +1646,9 @@ int intception_b200_last_fp32_rejections(void) {
 int intception_b200_last_hrr_redo(void) {
   Context* c = nullptr;
   if (get_context(&c)) return -1;
-  if (!c->last_redo) return c->host_redo;
-  IB_CUDA(cudaDeviceSynchronize());
+  std::lock_guard<std::mutex> lk(c->mu);
   int total = 0;
-  for (int g = 0; g < c->redo_groups; ++g) {
-    int h[2] = {0, 0};  // heavy and light counts
-    IB_CUDA(cudaMemcpy(h, c->last_redo + (size_t)g * c->redo_stride, 2 * sizeof(int), cudaMemcpyDeviceToHost));
-    total += h[0] + h[1];
-  }
+  IB_CUDA(c->read_redo(&total));
   return total;
 }
 
@@ -1671,6 +1733,7 @@ int intception_b200_batch_status(void) {
   Context* c = nullptr;
   int st = get_context(&c);
   if (st) return st;
+  std::lock_guard<std::mutex> lk(c->mu);
   int h = 0;
   IB_CUDA(cudaDeviceSynchronize());
   if (!c->last_status) return c->host_status;

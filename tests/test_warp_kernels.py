@@ -105,3 +105,28 @@ def test_status_after_graph_replay(nq, between):
     good.compute()
     assert good.device_status() == 0
     g.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('lmax', [2, 3])
+def test_graph_replay_after_larger_batches(lmax):
+    """A graph replays on the work buffers it was captured with: batches of more
+    quartets and of a higher l in between move the library on to larger ones.
+    Same kernels on the same inputs in a fixed order: the same bits; the counts
+    are the replayed batch's, also once the graph is closed."""
+    import torch
+    eng = eri.EriEngine(basis.independent_quartet_batch(8, 400, list(range(lmax + 1)), [4, 6], 0.01, 1e5, 4.0, True))
+    out = torch.empty(eng.out_size, dtype=torch.float64, device='cuda')
+    g = eng.graph(out)
+    ref, redo = eng.compute().cpu().numpy(), eri.last_hrr_redo()
+    assert redo > 0
+    for nq, l in ((5000, 2), (20000, 4)):
+        big = eri.EriEngine(basis.independent_quartet_batch(9, nq, [0, 1, l], [1, 2], 0.1, 60.0, 6.0, True))
+        big.compute()
+        out.fill_(7.0)
+        g.launch()
+        assert np.array_equal(out.cpu().numpy(), ref)
+        assert eri.last_hrr_redo() == redo and eng.device_status() == 0 and eng.fp32_rejected() == 0
+    g.close()
+    assert eri.last_hrr_redo() == redo
+    assert np.array_equal(eng.compute().cpu().numpy(), ref)
