@@ -607,9 +607,17 @@ __host__ __device__ inline constexpr double ib_rn_norm(int n) {
        : n == 9 ? 466.71786414003641 : n == 10 ? 1097.8288726985819 : n == 11 ? 2696.1716819638506
        : 6889.8632213814936;
 }
+// C(n, k), n <= 6, by products: a recursive form is called at run time where a
+// loop over k is not folded, and the stack of recursive calls is in no kernel's
+// stack size (it ran over the end of the local memory of the kernels whose own
+// frame is larger than the driver's default of 1 KB).
 __host__ __device__ inline constexpr double ib_binom(int n, int k) {
-  return k == 0 || k == n ? 1.0 : ib_binom(n - 1, k - 1) + ib_binom(n - 1, k);
+  const int m = k < n - k ? k : n - k;
+  return m == 0 ? 1.0 : m == 1 ? n : m == 2 ? n * (n - 1) / 2 : n * (n - 1) * (n - 2) / 6;
 }
+static_assert(ib_binom(6, 3) == 20.0 && ib_binom(6, 4) == 15.0 && ib_binom(5, 2) == 10.0 && ib_binom(3, 2) == 3.0 &&
+                  ib_binom(2, 2) == 1.0 && ib_binom(0, 0) == 1.0,
+              "binomial coefficients");
 // largest sum of |Cartesian coefficients| of one spherical function of the
 // library's transformation matrices, l = 0..6 (rounded up)
 __host__ __device__ inline constexpr double ib_sph_colsum(int l) {
