@@ -130,3 +130,21 @@ def test_graph_replay_after_larger_batches(lmax):
     g.close()
     assert eri.last_hrr_redo() == redo
     assert np.array_equal(eng.compute().cpu().numpy(), ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('sph', [False, True])
+@pytest.mark.parametrize('lmax', [1, 2])
+def test_every_quartet_of_batches_at_the_path_limits(sph, lmax):
+    """Every block of the batches either side of the path limits, the last
+    quartet's among them, against the oracle (out starts from 7, which no
+    evaluated element keeps)."""
+    import torch
+    b = basis.independent_quartet_batch(32, 3073, list(range(lmax + 1)), [1, 2, 3, 5], 0.1, 60.0, 6.0, sph)
+    ref = loader.oracle_batch(b, basis.sph_matrices(6))
+    for nq in (1, 296, 297, 3072, 3073):
+        eng = eri.EriEngine(b.subset(np.arange(nq)))
+        out = torch.full((eng.out_size,), 7.0, dtype=torch.float64, device='cuda')
+        got = eng.compute(out=out).cpu().numpy()
+        assert eng.out_size == b.out_off[nq - 1] + np.prod(b.block_dims(nq - 1))
+        assert np.abs(got - ref[:eng.out_size]).max() <= tolerance(ref), nq
