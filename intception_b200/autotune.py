@@ -89,6 +89,8 @@ def tune(nq=40000, reps=5, classes=None, log=print):
             eng._tune_bounds = torch.ones(b.nq, dtype=torch.float64, device='cuda')
             out = torch.empty(b.out_size, dtype=torch.float64, device='cuda')
             for prec in precs:
+                if len(precs) == 2:  # the class's FP32 kernel, whatever the built-in default
+                    eri.set_class_fp32(prec == eri.PREC_MIXED, cls)
                 v4 = (2 if prec == eri.PREC_MIXED else 0) + (1 if sph else 0)
                 times = []
                 for mi, mb in enumerate(MINB_VALUES):
@@ -101,6 +103,7 @@ def tune(nq=40000, reps=5, classes=None, log=print):
             del eng, out
         # the FP32 tier uses this class's FP32 kernel only where it beats FP64
         if len(precs) == 2:
+            eri.set_class_fp32(None, cls)
             ent['fp32'] = bool(min(ent['ms']['fp32_sph']) < FP32_GAIN * min(ent['ms']['fp64_sph']) and
                                min(ent['ms']['fp32_cart']) < FP32_GAIN * min(ent['ms']['fp64_cart']))
         else:  # FP64 kernels only: the FP32 slots take the FP64 choice

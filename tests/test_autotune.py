@@ -3,6 +3,8 @@ chain-order builds, and the tables the build bakes from the result."""
 import json
 import os
 
+import pytest
+
 from intception_b200 import autotune
 from intception_b200.emit import eri_emitter
 
@@ -42,3 +44,29 @@ def test_committed_tuning_covers_every_tuned_class():
     for ent in tun.values():
         assert len(ent['minb']) == 4 and all(0 <= m < len(autotune.MINB_VALUES) for m in ent['minb'])
         assert ent['order'] in ('dfs', 'level') and isinstance(ent['fp32'], bool)
+
+
+@pytest.mark.gpu
+def test_tuner_times_the_fp32_kernels(monkeypatch):
+    """The FP32 columns are of the FP32 kernel even where the built-in default
+    has it off: its result differs from the FP64 kernel's (by 2^-24 of the
+    intermediates, so by far more than FP64 rounding)."""
+    from intception_b200 import eri
+    out, rel = {}, []
+
+    def fake(eng, o, precision, reps, warmup=2):
+        kw = dict(bounds=eng._tune_bounds, skip_below=0.0, fp32_below=2.0, mixed_tol=1e300)
+        eng.compute(out=o, precision=precision, **(kw if precision == eri.PREC_MIXED else {}))
+        r = o.cpu()
+        if precision == eri.PREC_FP64:
+            out['ref'] = r
+        else:
+            rel.append(float((r - out['ref']).abs().max() / out['ref'].abs().max()))
+        return 1.0
+    monkeypatch.setattr(autotune, 'time_variant', fake)
+    try:
+        autotune.tune(nq=400, reps=1, classes=[(2, 1, 1, 1)], log=lambda *a: None)
+    finally:
+        for v4 in range(4):
+            eri.set_class_minb((2, 1, 1, 1), v4, 0)
+    assert len(rel) == 2 * len(autotune.MINB_VALUES) and all(1e-12 < x < 1e-4 for x in rel), rel
