@@ -428,7 +428,7 @@ __device__ __forceinline__ void ib2_overlap_pair(double xa, const double* __rest
 
 // Block-cooperative chunks: a block stages IB2_CHUNK pairs' inputs in shared
 // memory (coalesced, each input byte read once), sorts them by class there
-// (ballots; no atomics), and its warps run the sorted list, so that nearly all
+// (lane matches; no atomics), and its warps run the sorted list, so that nearly all
 // lanes of a warp execute the same unrolled class code.  Pairs of the
 // lane-group kernel and refused pairs are left out of the list.
 //
@@ -439,16 +439,20 @@ __device__ __forceinline__ void ib2_overlap_pair(double xa, const double* __rest
 //
 // The inputs of a complete chunk are contiguous byte ranges of the caller's
 // arrays; they are fetched by bulk copies (TMA, cp.async.bulk) with completion
-// counted on an mbarrier, issued as soon as the previous chunk is evaluated:
-// they arrive while its results are copied out and while the other block of
-// the SM evaluates.  The last (partial) chunk, and callers whose arrays are
-// not 16-byte aligned, take plain loads.
+// counted on an mbarrier.  The last (partial) chunk, and callers whose arrays
+// are not 16-byte aligned, take plain loads.
 //
-// 4e6 pairs, l <= 2, one B200: overlap 308 -> 162 us (105 at the HBM rate), nuclear
-// 288 -> 218 us (119), against a lane storing its own elements, 8-byte Boys
-// reads and a class sort by shared-memory atomics.  Above the HBM time is what
-// runs between the block's barriers at 16 warps an SM: the sort, the
-// recurrences (with a Boys row gather, nuclear) and the copy out.
+// Two forms, by the batch's lmax.  STAGED (lmax = 2): the results' stage takes
+// the room of a second input buffer, so a chunk's copies are issued when the
+// previous one is evaluated and arrive while its results are copied out.  The
+// other (lmax <= 1, where the blocks are short and their direct stores cheap;
+// lmax >= 3, where the pairs left to the lane-group kernel break the runs) has
+// two input buffers, the next chunk's copies in flight during the evaluation.
+// us for 4e6 pairs, without | with the stage, on one B200: overlap l = 0
+// 62 | 99, l <= 1 105 | 127, l <= 2 314 | 159 (105 at the HBM rate), nuclear
+// 94 | 124, 139 | 163 and 289 | 217 (119).  Above the HBM time is what runs
+// between the block's barriers at 16 warps an SM: the sort, the recurrences
+// (with a Boys row gather, nuclear) and the copy out.
 #define IB2_CHUNK 512
 #define IB2_TPB 256
 #define IB2_WR (IB2_CHUNK / 32)  // warp rounds of a chunk
@@ -464,11 +468,11 @@ struct Ib2Buf {
   int la[IB2_CHUNK], lb[IB2_CHUNK];
 };
 
-template <int KIND>
+template <int KIND, bool STAGED>
 struct Ib2Stage {
-  Ib2Buf<KIND> buf;
-  double out[IB2_OUT];
-  unsigned long long full;    // mbarrier: complete when a chunk's bulk copies have landed
+  Ib2Buf<KIND> buf[STAGED ? 1 : 2];
+  double out[STAGED ? IB2_OUT : 2];
+  unsigned long long full[2];  // mbarrier of each buffer: complete when a chunk's bulk copies have landed
   short order[IB2_CHUNK];     // chunk-local pair index, sorted by class
   unsigned char cls[IB2_CHUNK];
   unsigned char swp[IB2_CHUNK];
@@ -565,34 +569,41 @@ __device__ __forceinline__ void ib2_thread_pair(const Ib2Buf<KIND>& st, const un
   }
 }
 
-template <int KIND>
+template <int KIND, bool STAGED>
 __global__ void __launch_bounds__(IB2_TPB, 2) ib2_thread_kernel(const Ib2Args a) {
   constexpr int kClasses = KIND == 0 ? (IB2_LT + 1) * (IB2_LT + 1) : (IB2_LT + 1) * (IB2_LT + 2) / 2;
   constexpr int kRounds = IB2_CHUNK / IB2_TPB;
   extern __shared__ __align__(16) unsigned char ib2_raw[];
-  Ib2Stage<KIND>& st = *reinterpret_cast<Ib2Stage<KIND>*>(ib2_raw);
-  Ib2Buf<KIND>& bf = st.buf;
+  Ib2Stage<KIND, STAGED>& st = *reinterpret_cast<Ib2Stage<KIND, STAGED>*>(ib2_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long nchunk = ((long long)a.n + IB2_CHUNK - 1) / IB2_CHUNK;
   const long long nfull = a.bulk_ok ? (long long)a.n / IB2_CHUNK : 0;  // chunks fetched by bulk copies
-  const unsigned mb = ib2_smem_addr(&st.full);
+  const unsigned mb0 = ib2_smem_addr(&st.full[0]), mb1 = ib2_smem_addr(&st.full[1]);
   if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb0) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb1) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if ((long long)blockIdx.x < nfull) ib2_issue<KIND>(a, bf, blockIdx.x, mb);
+    if ((long long)blockIdx.x < nfull) ib2_issue<KIND>(a, st.buf[0], blockIdx.x, mb0);
   }
   __syncthreads();
   int k = 0;
   for (long long ch = blockIdx.x; ch < nchunk; ch += gridDim.x, ++k) {
     const long long nxt = ch + gridDim.x;
+    const int b = STAGED ? 0 : k & 1, use = STAGED ? k : k >> 1;  // this chunk's buffer, and which of its uses
+    Ib2Buf<KIND>& bf = st.buf[b];
+    const unsigned mb = b ? mb1 : mb0, mb_next = b ? mb0 : mb1;
+    // two buffers: fetch the next chunk into the other one (read by the
+    // previous iteration, which ended with a block barrier)
+    if (!STAGED && threadIdx.x == 0 && nxt < nfull) ib2_issue<KIND>(a, st.buf[STAGED ? 0 : b ^ 1], nxt, mb_next);
     const int p0 = (int)(ch * IB2_CHUNK);
     const int np = min(IB2_CHUNK, a.n - p0);
     if (ch < nfull) {
-      const bool ok = ib2_wait(mb, k & 1, a.wait_iters);
-      if (__syncthreads_or(!ok)) {  // uniform: report, drain this chunk's copies (the only ones in flight), stop
+      const bool ok = ib2_wait(mb, use & 1, a.wait_iters);
+      if (__syncthreads_or(!ok)) {  // uniform: report, drain the copies still in flight, stop
         if (threadIdx.x == 0) {
           if (a.status) atomicExch(a.status, IB_ERR_TIMEOUT);
-          ib2_wait(mb, k & 1, a.wait_iters);
+          ib2_wait(mb, use & 1, a.wait_iters);
+          if (!STAGED && nxt < nfull) ib2_wait(mb_next, ((k + 1) >> 1) & 1, a.wait_iters);
         }
         return;
       }
@@ -631,27 +642,35 @@ __global__ void __launch_bounds__(IB2_TPB, 2) ib2_thread_kernel(const Ib2Args a)
           st.swp[t] = la < lb;
         }
         st.cls[t] = (unsigned char)c;
-        const long long end = bf.off[t] + (c == 255 ? 0 : ib2_ncart(la) * ib2_ncart(lb));
-        run = run && c != 255 && (t + 1 < np ? bf.off[t + 1] == end : end - bf.off[0] <= IB2_OUT);
+        if (STAGED) {
+          const long long end = bf.off[t] + (c == 255 ? 0 : ib2_ncart(la) * ib2_ncart(lb));
+          run = run && c != 255 && (t + 1 < np ? bf.off[t + 1] == end : end - bf.off[0] <= IB2_OUT);
+        }
       }
       cl[q] = c;
-      rk[q] = 0;
-#pragma unroll
-      for (int v = 0; v < kClasses; ++v) {
-        const unsigned bal = __ballot_sync(0xffffffffu, c == v);
-        if (c == v) rk[q] = __popc(bal & ((1u << lane) - 1u));
-        if (lane == v) st.cnt[wr][v] = __popc(bal);
-      }
+      if (lane < 16) st.cnt[wr][lane] = 0;
+      const unsigned same = __match_any_sync(0xffffffffu, c);
+      rk[q] = __popc(same & ((1u << lane) - 1u));
+      __syncwarp();
+      if (c != 255 && rk[q] == 0) st.cnt[wr][c] = __popc(same);
     }
-    const bool staged = __syncthreads_and(run);
+    bool staged = false;
+    if (STAGED)
+      staged = __syncthreads_and(run);
+    else
+      __syncthreads();
     if (warp == 0) {
       int n = 0;
-      if (lane < kClasses)
+      if (lane < kClasses) {
+        int v[IB2_WR];
+#pragma unroll
+        for (int w = 0; w < IB2_WR; ++w) v[w] = st.cnt[w][lane];
+#pragma unroll
         for (int w = 0; w < IB2_WR; ++w) {
-          const int v = st.cnt[w][lane];
           st.cnt[w][lane] = n;
-          n += v;
+          n += v[w];
         }
+      }
       int s = n;
       for (int o = 1; o < 16; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, s, o);
@@ -669,16 +688,22 @@ __global__ void __launch_bounds__(IB2_TPB, 2) ib2_thread_kernel(const Ib2Args a)
     const int total = st.start[kClasses];
     const long long o0 = bf.off[0];
     // units of 32 pairs in ascending class (cost) order; warp w takes unit w and
-    // unit IB2_WR - 1 - w, so that the warps' shares are alike at the barrier
+    // the w-th unit from the end, so that the warps' shares are alike at the barrier
+    static_assert(kRounds == 2, "each warp takes two units");
+    const int last = (total + 31) / 32 - 1;
 #pragma unroll 1
     for (int q = 0; q < kRounds; ++q) {
-      const int i = 32 * (q & 1 ? (q + 1) * (IB2_TPB / 32) - 1 - warp : q * (IB2_TPB / 32) + warp) + lane;
-      if (i >= total) continue;
+      const int u = q == 0 ? warp : last - warp, i = 32 * u + lane;
+      if (i >= total || (q == 1 && u < IB2_TPB / 32)) continue;
       const int j = st.order[i];
-      if (staged)
+      if (STAGED && staged)
         ib2_thread_pair<KIND>(bf, st.swp, st.cls[j], j, a.rows, st.out + (int)(bf.off[j] - o0));
       else
         ib2_thread_pair<KIND>(bf, st.swp, st.cls[j], j, a.rows, a.out + bf.off[j]);
+    }
+    if (!STAGED) {
+      __syncthreads();  // this buffer and the sort arrays are reused
+      continue;
     }
     const int nout = staged ? (int)(bf.off[np - 1] - o0) + ib2_ncart(bf.la[np - 1]) * ib2_ncart(bf.lb[np - 1]) : 0;
     __syncthreads();  // the inputs are read, the results staged
@@ -778,8 +803,10 @@ int twoidx_setup(TwoIdxDevice** out) {
     ok = ok && cudaGetSymbolAddress((void**)&d.single, ib2_single) == cudaSuccess;
     ok = ok && cudaGetSymbolAddress((void**)&d.single_out, ib2_single_out) == cudaSuccess;
     ok = ok && cudaGetSymbolAddress((void**)&d.single_status, ib2_single_status) == cudaSuccess;
-    ok = ok && allow_smem(ib2_thread_kernel<0>, sizeof(Ib2Stage<0>)) == cudaSuccess;
-    ok = ok && allow_smem(ib2_thread_kernel<1>, sizeof(Ib2Stage<1>)) == cudaSuccess;
+    ok = ok && allow_smem(ib2_thread_kernel<0, true>, sizeof(Ib2Stage<0, true>)) == cudaSuccess;
+    ok = ok && allow_smem(ib2_thread_kernel<0, false>, sizeof(Ib2Stage<0, false>)) == cudaSuccess;
+    ok = ok && allow_smem(ib2_thread_kernel<1, true>, sizeof(Ib2Stage<1, true>)) == cudaSuccess;
+    ok = ok && allow_smem(ib2_thread_kernel<1, false>, sizeof(Ib2Stage<1, false>)) == cudaSuccess;
     // each group size serves the lmax values pick_group maps to it
     ok = ok && allow_smem(ib2_nuclear_kernel<32>, smem_bytes(1, 32, IB2_LMAX)) == cudaSuccess;
     ok = ok && allow_smem(ib2_nuclear_kernel<16>, smem_bytes(1, 16, 2)) == cudaSuccess;
@@ -820,10 +847,15 @@ int launch(int kind, const Ib2Args& a0, int nsm, cudaStream_t s) {
                  aligned16(a0.off) && aligned16(a0.la) && aligned16(a0.lb) && (kind == 0 || aligned16(a0.cc));
     const long long chunks = ((long long)a0.n + IB2_CHUNK - 1) / IB2_CHUNK;
     const int grid = (int)std::max(1LL, std::min<long long>(chunks, 2LL * nsm));
-    if (kind == 0)
-      ib2_thread_kernel<0><<<grid, IB2_TPB, sizeof(Ib2Stage<0>), s>>>(at);
+    const bool staged = a0.lmax == IB2_LT;
+    if (kind == 0 && staged)
+      ib2_thread_kernel<0, true><<<grid, IB2_TPB, sizeof(Ib2Stage<0, true>), s>>>(at);
+    else if (kind == 0)
+      ib2_thread_kernel<0, false><<<grid, IB2_TPB, sizeof(Ib2Stage<0, false>), s>>>(at);
+    else if (staged)
+      ib2_thread_kernel<1, true><<<grid, IB2_TPB, sizeof(Ib2Stage<1, true>), s>>>(at);
     else
-      ib2_thread_kernel<1><<<grid, IB2_TPB, sizeof(Ib2Stage<1>), s>>>(at);
+      ib2_thread_kernel<1, false><<<grid, IB2_TPB, sizeof(Ib2Stage<1, false>), s>>>(at);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return IB_ERR_CUDA;
   }

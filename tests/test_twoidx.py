@@ -291,3 +291,41 @@ def test_bounded_wait_gives_up_and_reports_timeout(kind):
     torch.cuda.synchronize()
     assert batch.device_status() == 0
     _assert_blocks(out.cpu().numpy(), ref, pairs, 1e-12)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('kind', [0, 1])
+@pytest.mark.parametrize('lmax', [1, 2, 3])
+@pytest.mark.parametrize('place', ['packed', 'reversed', 'gapped', 'grouped'])
+def test_output_placements(kind, lmax, place):
+    """Whole chunks and a remainder with the blocks placed one after the other,
+    in the opposite order, with gaps, and with the pairs grouped by class (runs
+    shorter and longer than a chunk's output stage): every block at its offset,
+    nothing between them."""
+    import torch
+    from intception_b200 import twoidx
+    from oracle import loader
+    n = 4 * 512 + 45
+    pairs = twoidx.make_pairs(n, lmax=lmax, seed=17)
+    if place == 'grouped':
+        order = np.argsort(10 * pairs['la'] + pairs['lb'], kind='stable')
+        pairs = {k: v[order] for k, v in pairs.items()}
+    packed, size = twoidx.block_offsets(pairs['la'], pairs['lb'])
+    dims = np.diff(np.append(packed, size))
+    off = packed.copy()
+    if place == 'reversed':
+        off = size - packed - dims
+    if place == 'gapped':
+        off += 3 * (np.arange(n) // 700)
+        size = int(off[-1] + dims[-1])
+    in_order = dict(pairs, off=packed, size=int(dims.sum()))
+    ref = loader.twoidx_batch(kind, in_order)
+    tb = twoidx.TwoIndexBatch(dict(pairs, off=off, size=size))
+    out = torch.full((size,), -7.0, dtype=torch.float64, device='cuda')
+    got = tb.compute(kind, out=out).cpu().numpy()
+    assert tb.device_status() == 0
+    at = np.repeat(off - packed, dims) + np.arange(len(ref))
+    _assert_blocks(got[at], ref, in_order, 1e-12)
+    rest = np.ones(size, bool)
+    rest[at] = False
+    assert np.all(got[rest] == -7.0)
