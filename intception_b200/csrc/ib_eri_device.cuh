@@ -32,8 +32,10 @@
 #define IB_NCLASS (IB_NPAIR_EXT * (IB_NPAIR_EXT + 1) / 2)
 #define IB_BOYS_TAYLOR 7
 // ranges: FP64 and FP32 [begin, end) per class, three more pairs, then the end
-// of each class's FP64 quartets of at least 2^IB_MERGED_LONG_LOG2 primitive quartets
+// of each class's FP64 quartets of at least 2^IB_MERGED_LONG_LOG2 primitive
+// quartets, then [begin, end) of each class's short FP64 quartets
 #define IB_SLOT_LONG_END (4 * IB_NCLASS + 6)
+#define IB_SLOT_SHORT (IB_SLOT_LONG_END + IB_NCLASS)
 #define IB_MERGED_LONG_LOG2 7
 
 struct IbItem {
@@ -297,7 +299,7 @@ __device__ __forceinline__ int ib_reverse_for_classes(const int* __restrict__ sh
   return 1;
 }
 
-// Per-lane constants of a FP32 lane-group kernel.  steps: the lane's base-chain
+// Per-lane constants of a lane-group kernel.  steps: the lane's base-chain
 // path, 5 bits per step (direction 0..2, or 3 for an identity step that pads
 // shorter paths at the front; then the exponent before the step); misc: the
 // lane's Cartesian component (3 bits per axis) and the lanes owning
@@ -386,9 +388,46 @@ struct IbClassEntry {
   IbLaunchFn launch;    // null: no unrolled kernel (the generic kernel serves the class)
   IbOccFn occupancy;
   int kind;             // 1: FP64 variants only, 2: FP64 and FP32 variants
+  // FP64 kernel of the class's short quartets (variant 0 Cartesian, 1
+  // spherical; null: none): floor(log2(primitive quartets)) <= short_log2
+  IbLaunchFn short_launch;
+  IbOccFn short_occupancy;
+  int short_log2;
 };
 
 __host__ __device__ inline constexpr double ib_two_pi52() { return 34.98683665524972497; }  // 2 pi^(5/2)
+
+// F_m(T), m = 0..L, for the FP64 lane-group kernels, from the full table (rows
+// of IB_BOYS_NCOL values F_n(T_i); columns L..L+6 of one row).
+template <int L>
+__device__ __forceinline__ void ib_boys(double T, const double* __restrict__ tab, double* F) {
+  if (T < IB_BOYS_TMAX) {
+    const int i = __double2int_rn(T * (double)IB_BOYS_H_INV);
+    const double dx = (double)i * (1.0 / IB_BOYS_H_INV) - T;
+    const double* r = tab + i * IB_BOYS_NCOL + L;
+    double f = __ldg(r + 6) * (1.0 / 720.0);
+    f = fma(f, dx, __ldg(r + 5) * (1.0 / 120.0));
+    f = fma(f, dx, __ldg(r + 4) * (1.0 / 24.0));
+    f = fma(f, dx, __ldg(r + 3) * (1.0 / 6.0));
+    f = fma(f, dx, __ldg(r + 2) * 0.5);
+    f = fma(f, dx, __ldg(r + 1));
+    f = fma(f, dx, __ldg(r));
+    F[L] = f;
+    if (L > 0) {
+      const double e = exp(-T), t2 = T + T;
+#pragma unroll
+      for (int m = L - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], e) * (1.0 / (2 * m + 1));
+    }
+  } else {
+    const double oT = 1.0 / T;
+    F[0] = sqrt(0.78539816339744830962 * oT);  // (1/2) sqrt(pi/T)
+    if (L > 0) {
+      const double he = 0.5 * exp(-T);
+#pragma unroll
+      for (int m = 0; m < L; ++m) F[m + 1] = fma((double)m + 0.5, F[m], -he) * oT;
+    }
+  }
+}
 
 // F_m(T), m = 0..L, for the FP32 tier's setup: 7-term Taylor about the nearest
 // table row and downward recursion, above the table's end the asymptotic F_0
@@ -541,14 +580,15 @@ __device__ __forceinline__ double ib_pair_factor(double xa, double ca, double xb
   return ca * cb * exp(-xa * xb * oz * r2);
 }
 
-// Bra pair of primitives ia, ib for the FP32 tier: the reciprocal by
+// Bra pair of primitives ia, ib.  F32SETUP (the FP32 tier): the reciprocal by
 // ib_rcp_refined and the prefactor by ib_pair_factor_f32.
+template <bool F32SETUP>
 __device__ __forceinline__ void ib_bra_pair(const IbLaunch& a, const IbQuartet& g, int ia, int ib, IbBraPair& bp) {
   const double xa = __ldg(a.prim_exp + g.ptr[0] + ia), ca = __ldg(a.prim_coef + g.ptr[0] + ia);
   const double xb = __ldg(a.prim_exp + g.ptr[1] + ib), cb = __ldg(a.prim_coef + g.ptr[1] + ib);
   bp.zeta = xa + xb;
-  bp.oz = ib_rcp_refined(bp.zeta);
-  bp.K = ib_pair_factor_f32(xa, ca, xb, cb, bp.oz, g.RAB2);
+  bp.oz = F32SETUP ? ib_rcp_refined(bp.zeta) : 1.0 / bp.zeta;
+  bp.K = F32SETUP ? ib_pair_factor_f32(xa, ca, xb, cb, bp.oz, g.RAB2) : ib_pair_factor(xa, ca, xb, cb, bp.oz, g.RAB2);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     bp.P[d] = (xa * g.A[d] + xb * g.B[d]) * bp.oz;
@@ -1017,13 +1057,14 @@ __device__ __forceinline__ bool ib_prim_quartet(const IbLaunch& a, const IbQuart
                                                 IbPrimQuartet<R>& pq) {
   const double xc = __ldg(a.prim_exp + g.ptr[2] + ic), cc = __ldg(a.prim_coef + g.ptr[2] + ic);
   const double xd = __ldg(a.prim_exp + g.ptr[3] + id), cd = __ldg(a.prim_coef + g.ptr[3] + id);
-  // reciprocals, exponentials, square root and Boys values in float
-  // (reciprocals refined in FP64); the error bound counts
-  // IB_F32_SETUP_ROUNDINGS more roundings for the scaled F_m
-  const double eta = xc + xd, oe = ib_rcp_refined(eta);
-  const double Kcd = ib_pair_factor_f32(xc, cc, xd, cd, oe, g.RCD2);
+  // the FP32 tier (R = float) computes the reciprocals, exponentials, square
+  // root and Boys values in float (reciprocals refined in FP64); its error
+  // bound counts IB_F32_SETUP_ROUNDINGS more roundings for the scaled F_m
+  constexpr bool F32 = sizeof(R) == 4;
+  const double eta = xc + xd, oe = F32 ? ib_rcp_refined(eta) : 1.0 / eta;
+  const double Kcd = F32 ? ib_pair_factor_f32(xc, cc, xd, cd, oe, g.RCD2) : ib_pair_factor(xc, cc, xd, cd, oe, g.RCD2);
   if (bp.K * Kcd == 0.0) return false;
-  const double ozpe = ib_rcp_refined(bp.zeta + eta);
+  const double ozpe = F32 ? ib_rcp_refined(bp.zeta + eta) : 1.0 / (bp.zeta + eta);
   const double rho = bp.zeta * eta * ozpe;
   double Q[3], PQ[3];
 #pragma unroll
@@ -1032,8 +1073,11 @@ __device__ __forceinline__ bool ib_prim_quartet(const IbLaunch& a, const IbQuart
     PQ[d] = bp.P[d] - Q[d];
   }
   const double RPQ2 = PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2];
-  ib_boys_f32<L>(rho * RPQ2, boys_tab, F);
-  const double pref = ib_two_pi52() * bp.oz * oe * (double)sqrtf((float)ozpe) * bp.K * Kcd;
+  if (F32)
+    ib_boys_f32<L>(rho * RPQ2, boys_tab, F);
+  else
+    ib_boys<L>(rho * RPQ2, boys_tab, F);
+  const double pref = ib_two_pi52() * bp.oz * oe * (F32 ? (double)sqrtf((float)ozpe) : sqrt(ozpe)) * bp.K * Kcd;
 #pragma unroll
   for (int m = 0; m <= L; ++m) F[m] *= pref;
 #pragma unroll

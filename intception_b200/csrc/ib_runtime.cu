@@ -49,8 +49,8 @@ constexpr int kSlotFp32 = 2 * IB_NCLASS;        // ranges offset of the FP32 cop
 constexpr int kSlotGenHeavy = 4 * IB_NCLASS;    // [begin, end) of the generic kernel's heavy quartets
 constexpr int kSlotSkip = 4 * IB_NCLASS + 2;    // [begin, end) of the screened-out quartets
 constexpr int kSlotGenLight = 4 * IB_NCLASS + 4;  // [begin, end) of the generic kernel's light quartets
-constexpr int kNRanges = IB_SLOT_LONG_END + IB_NCLASS;
-constexpr int kNCounters = 3 * IB_NCLASS;      // quartet counters: FP64 pass, FP32 pass, FP64 recheck pass
+constexpr int kNRanges = IB_SLOT_SHORT + 2 * IB_NCLASS;
+constexpr int kNCounters = 4 * IB_NCLASS;  // quartet counters: FP64 pass, FP32 pass, FP64 recheck pass, short quartets
 // sort key: skip(1) generic(1) fp32(1) class(9) work(4), two radix passes; a
 // generic quartet's class and work bits hold light(1) and its cost code (8)
 constexpr int kKeyBits = 16;
@@ -65,6 +65,18 @@ constexpr size_t kScratchCap = size_t(4) << 30;  // bytes of generic-kernel scra
 // launches and as fast from 600 quartets on.
 constexpr int kSmallBatch = 296;
 constexpr int kMergedBatch = 3072;
+// Quartets with few primitive quartets go to the classes' lane-group kernels
+// (IB_SLOT_SHORT) in batches that evaluate at least this many, by the mean
+// contraction length of the basis: below, the warp kernels' latency hides and
+// the extra launches and shorter ranges cost more.  Step without / with them:
+// K = 1 50 000 quartets l <= 1 190 / 149 us, l <= 2 331 / 279 (12 000: 251 /
+// 232); K 1..3 50 000 524 / 619, 100 000 l <= 1 323 / 285, l <= 2 879 / 877,
+// 6e5 3.48 / 2.94 ms; K 1..6 100 000 548 / 568, 3e5 915 / 879 (l <= 2 2.13 /
+// 2.17 ms), 1e6 7.54 / 7.41 ms.
+int short_batch(const intception_b200_basis* b) {
+  const double k = b->nshell > 0 ? (double)b->nprim / b->nshell : 1e9;
+  return k <= 1.6 ? (b->lmax <= 1 ? 1 << 13 : 1 << 15) : k <= 2.25 ? 3 << 15 : 1 << 18;
+}
 constexpr int kRedoGroups = 4;  // redo lists of an l >= 3 batch (dispatch)
 constexpr int kTickets = 2 * (1 + kRedoGroups);  // generic-kernel ticket pairs: the range launch, each redo list
 // blocks per cluster sharing a heavy generic quartet: a redo list is short and
@@ -154,7 +166,7 @@ struct Context {
   cudaStream_t side[kNSideMax] = {};
   cudaEvent_t fork = nullptr, join[kNSideMax] = {};
   DevBuf boys_tab, rys_tab, boys_row, sph, keys, vals, keys2, vals2, items, ranges, cub_tmp, scratch;
-  DevBuf counters;  // per class kernel launch of a batch: the next quartet (FP64, FP32, FP64 recheck passes)
+  DevBuf counters;  // per class kernel launch of a batch: the next quartet (kNCounters)
   DevBuf sw_quartets, sw_sizes, sw_off, sw_tmp, sw_blocks;  // Schwarz-bound work buffers
   std::vector<int> classes;  // emitted class ids, the heaviest first (descending id)
   std::vector<int> lmax_of;  // their largest l
@@ -225,6 +237,8 @@ struct Context {
   }
   IbClassEntry table[IB_NCLASS] = {};
   int occ[IB_NCLASS][4 * IB_NMINB] = {};
+  int short_occ[IB_NCLASS][2] = {};
+  DevBuf short_log2;  // per class: IbClassEntry::short_log2 (-1: no kernel for short quartets)
   int minb_idx[IB_NCLASS][4] = {};  // register budget chosen per class and variant (autotuned defaults)
   std::mutex mu;
 };
@@ -316,7 +330,10 @@ __global__ void ib_build_items(const unsigned* __restrict__ keys, const int* __r
                                const int* __restrict__ shell_k, const int* __restrict__ shell_ptr,
                                const double* __restrict__ prim_exp, const double* __restrict__ shell_xyz,
                                const long long* __restrict__ out_off, int spherical, int route_rev,
-                               IbItem* __restrict__ items, int* __restrict__ ranges) {
+                               const int* __restrict__ short_log2, int short_min, IbItem* __restrict__ items,
+                               int* __restrict__ ranges) {
+  // screened quartets sort last: at least short_min quartets are evaluated
+  if (short_log2 && (keys[short_min - 1] >> 15)) short_log2 = nullptr;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nq; p += gridDim.x * blockDim.x) {
     const int q = order[p];
     int s[4], l[4], n[4];
@@ -357,9 +374,14 @@ __global__ void ib_build_items(const unsigned* __restrict__ keys, const int* __r
       continue;
     }
     const int cid = slot & 511, fp32 = (slot >> 9) & 1;
-    const int rs = 2 * (cid + fp32 * IB_NCLASS);
-    if (prev != slot) ranges[rs] = p;
-    if (next != slot) ranges[rs + 1] = p + 1;
+    // primitive quartet counts descend in a class: its short quartets come last
+    const int sl = short_log2 && !fp32 ? short_log2[cid] : -1;
+    const bool is_short = 15 - (int)(key & 15u) <= sl;
+    const bool begins = prev != slot || (15 - (int)(keys[p - 1] & 15u) <= sl) != is_short;
+    const bool ends = next != slot || (15 - (int)(keys[p + 1] & 15u) <= sl) != is_short;
+    const int rs = is_short ? IB_SLOT_SHORT + 2 * cid : 2 * (cid + fp32 * IB_NCLASS);
+    if (begins) ranges[rs] = p;
+    if (ends) ranges[rs + 1] = p + 1;
     // key bits 0-3: 15 - log2 of the primitive quartet count, ascending in a class
     const unsigned lim = 15 - IB_MERGED_LONG_LOG2;
     if (!fp32 && (key & 15u) <= lim && (next != slot || (keys[p + 1] & 15u) > lim)) ranges[IB_SLOT_LONG_END + cid] = p + 1;
@@ -627,7 +649,7 @@ int get_context(Context** out) {
     IB_CUDA(c->sph.ensure(sph.size() * sizeof(double)));
     IB_CUDA(cudaMemcpy(c->sph.p, sph.data(), sph.size() * sizeof(double), cudaMemcpyHostToDevice));
     IB_CUDA(c->ranges.ensure(kNRanges * sizeof(int)));
-    IB_CUDA(c->counters.ensure((kNCounters + 1) * sizeof(int)));  // + the drop-in's own
+    IB_CUDA(c->counters.ensure(kNCounters * sizeof(int)));
     IB_CUDA(c->tickets.ensure(kTickets * sizeof(int)));
     IB_CUDA(c->small_ctl.ensure((18 + 2 * (size_t)kSmallBatch) * sizeof(int)));
     c->status = c->small_ctl.as<int>();
@@ -644,6 +666,8 @@ int get_context(Context** out) {
       c->kind_h[cid] = kind[cid];
       c->fp32_classes += kind[cid] == 2;
       for (int v = 0; v < 4 * IB_NMINB; ++v) c->occ[cid][v] = std::max(1, c->table[cid].occupancy(v));
+      for (int v = 0; v < 2 && c->table[cid].short_launch; ++v)
+        c->short_occ[cid][v] = std::max(1, c->table[cid].short_occupancy(v));
       for (int v = 0; v < 4; ++v) c->minb_idx[cid][v] = std::min(std::max(ib_tuned_minb[cid][v], 0), IB_NMINB - 1);
       c->slice_cap[cid] = ib_tuned_slice_cap[cid];
     }
@@ -655,6 +679,11 @@ int get_context(Context** out) {
     if (const char* env = std::getenv("INTCEPTION_B200_SLICE_BOOST")) c->slice_boost = std::max(1, std::atoi(env));
     if (const char* env = std::getenv("INTCEPTION_B200_MAX_SLICES"))
       for (int cid = 0; cid < IB_NCLASS; ++cid) c->slice_cap[cid] = std::max(0, std::atoi(env));
+    std::vector<int> short_log2(IB_NCLASS, -1);
+    for (int cid = 0; cid < IB_NCLASS; ++cid)
+      if (c->table[cid].short_launch) short_log2[cid] = c->table[cid].short_log2;
+    IB_CUDA(c->short_log2.ensure(IB_NCLASS * sizeof(int)));
+    IB_CUDA(cudaMemcpy(c->short_log2.p, short_log2.data(), IB_NCLASS * sizeof(int), cudaMemcpyHostToDevice));
     IB_CUDA(c->kind.ensure(IB_NCLASS * sizeof(int)));
     IB_CUDA(cudaMemcpy(c->kind.p, kind.data(), IB_NCLASS * sizeof(int), cudaMemcpyHostToDevice));
     IB_CUDA(cudaGetLastError());
@@ -706,7 +735,7 @@ cudaError_t redo_launch(Context* c, cudaStream_t s, const IbLaunch& a, bool sph,
 // Launch the emitted kernels for the given variants and the generic kernel;
 // items/ranges already on the device.  Returns the number of kernels launched.
 int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, int nq, bool fp64_present, bool fp32_present, bool sph,
-             int lmax, int* nlaunch, const ZeroFill* zf = nullptr) {
+             int lmax, bool shorts, int* nlaunch, const ZeroFill* zf = nullptr) {
   // the generic kernel's tickets (zeroed by classify): pair 0 for its range launch, pair 1 + g for redo list g
   int* const tk = c->tickets.as<int>();
   // side streams: one per launch, up to nside (an l <= 2 batch needs 22 of the 40)
@@ -810,6 +839,20 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, int nq, bool fp64_pr
         c->table[cid].launch(vt64, c->nsm * c->occ[cid][vt64], ss, ar);
         ++k;
       }
+    }
+  }
+  if (fp64_present && shorts) {
+    IbLaunch as = a;
+    as.ranges = a.ranges + IB_SLOT_SHORT;
+    for (size_t ci = 0; ci < c->classes.size(); ++ci) {
+      const int cid = c->classes[ci];
+      if (c->lmax_of[ci] > lmax || !c->table[cid].short_launch) continue;
+      if (G > 1) as.redo = a.redo + (size_t)((k % nuse) % G) * c->redo_stride;
+      as.max_slices = c->slice_cap[cid];
+      as.counter = c->counters.as<int>() + 3 * IB_NCLASS + cid;
+      const int v = sph ? 1 : 0;
+      c->table[cid].short_launch(v, c->nsm * c->short_occ[cid][v], c->side[k % nuse], as);
+      ++k;
     }
   }
   if (generic && lmax < 3) IB_CUDA(launch_generic());
@@ -1285,6 +1328,8 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   IB_CUDA(cudaMemsetAsync(c->status, 0, sizeof(int), s));
   const IbZeroed zeroed = {c->ranges.as<int>(), c->counters.as<int>(), c->tickets.as<int>(), c->redo.as<int>(),
                            c->flags.as<int>(), kNRanges, kNCounters, kTickets, c->redo_groups, c->redo_stride};
+  const int short_min = short_batch(basis);
+  const bool shorts = nq >= short_min;
   const int grid = std::min((nq + 255) / 256, c->nsm * 16);
   const bool use_bounds = bounds != nullptr && (precision == IB_PREC_MIXED || skip_below > 0.0);
   ib_classify<<<grid, 256, 0, s>>>(quartets, basis->shell_l, basis->shell_k, basis->shell_ptr, basis->prim_exp,
@@ -1299,7 +1344,8 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
                                           c->vals.as<int>(), c->vals2.as<int>(), nq, 0, kKeyBits, s));
   ib_build_items<<<grid, 256, 0, s>>>(c->keys2.as<unsigned>(), c->vals2.as<int>(), nq, quartets, basis->shell_l,
                                       basis->shell_k, basis->shell_ptr, basis->prim_exp, basis->shell_xyz, out_off,
-                                      spherical ? 1 : 0, c->hrr_tol > 0.0 ? 0 : 1, c->items.as<IbItem>(),
+                                      spherical ? 1 : 0, c->hrr_tol > 0.0 ? 0 : 1,
+                                      shorts ? c->short_log2.as<int>() : nullptr, short_min, c->items.as<IbItem>(),
                                       c->ranges.as<int>());
   ++*nl;
   IB_CUDA(cudaGetLastError());
@@ -1320,7 +1366,7 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   a.hrr_tol = c->hrr_tol;
   if (precision == IB_PREC_MIXED) a.mixed_tol = mixed_tol;
   const ZeroFill zf = {c->keys.as<unsigned>(), nq, quartets, basis->shell_l, out_off};
-  return dispatch(c, s, a, nq, true, precision == IB_PREC_MIXED, spherical != 0, basis->lmax, nl,
+  return dispatch(c, s, a, nq, true, precision == IB_PREC_MIXED, spherical != 0, basis->lmax, shorts, nl,
                   use_bounds && skip_below > 0.0 ? &zf : nullptr);
 }
 }  // namespace

@@ -366,6 +366,26 @@ THREAD_TARGETS = 54
 ROTATED = {(1, 1, 1, 1), (2, 2, 1, 0), (3, 2, 1, 0)}
 
 
+# Quartets of at most 2^log2 (rounded down) primitive quartets stay with the
+# lane-group kernel (group_emitter.py), which puts several of them in a warp;
+# the warp kernels leave most lanes without a primitive quartet.  (largest
+# floor(log2) of the primitive quartet count, register budget): the last power
+# of two where the lane-group kernel was at least 4 % faster.  us per 4e5
+# quartets (the whole step, 1e5 with an f shell), lane group | warp, for 1, 4,
+# 16 and 36 primitive quartets: (ss|ss) 406|641 417|674 483|699 695|761,
+# (pp|pp) 613|1844 767|1942 1438|2336 2587|3037, (ds|ds) 497|1620 650|1704
+# 1254|1755 2289|2072, (dd|ds) 1169|2035 1653|2156 3472|3093, (dd|dp) 3128|2563;
+# for 1, 4 and 16: (fp|ps) 308|482 314|513 522|616, (fd|ds) 620|925 854|968
+# 1759|1321, (fs|dp) 651|472.
+SHORT = {(0, 0, 0, 0): (5, 1), (1, 0, 0, 0): (4, 0), (1, 0, 1, 0): (4, 1), (1, 1, 0, 0): (5, 1), (1, 1, 1, 0): (4, 0),
+         (1, 1, 1, 1): (4, 1), (2, 0, 0, 0): (4, 0), (2, 0, 1, 0): (4, 0), (2, 0, 1, 1): (4, 1), (2, 0, 2, 0): (4, 1),
+         (2, 1, 0, 0): (5, 1), (2, 1, 1, 0): (4, 0), (2, 1, 1, 1): (3, 1), (2, 1, 2, 0): (3, 1), (2, 2, 0, 0): (5, 1),
+         (2, 2, 1, 0): (4, 0), (2, 2, 1, 1): (3, 0), (2, 2, 2, 0): (3, 0),
+         (3, 0, 0, 0): (4, 1), (3, 0, 1, 0): (4, 1), (3, 0, 1, 1): (2, 0), (3, 0, 2, 0): (0, 0), (3, 1, 0, 0): (4, 1),
+         (3, 1, 1, 0): (4, 1), (3, 1, 1, 1): (2, 0), (3, 1, 2, 0): (2, 0), (3, 2, 0, 0): (4, 0), (3, 2, 1, 0): (4, 0),
+         (3, 2, 1, 1): (2, 0), (3, 2, 2, 0): (2, 0), (3, 3, 0, 0): (4, 0), (3, 3, 1, 0): (2, 0)}
+
+
 def fp64_emitter(c):
     from .warp_emitter import RotationEmitter, RysEmitter, ThreadEmitter
     if c in ROTATED:
@@ -404,19 +424,24 @@ def emitted_classes():
 def class_source(c, fp32):
     """CUDA source of class c (its kernels, launcher and occupancy query) and
     its statistics."""
-    from .group_emitter import GroupEmitter, launcher
+    from .group_emitter import GroupEmitter, MINB_VALUES, launcher, short_launcher
     e = fp64_emitter(c)
     parts = [e.kernel()]
     only = None if max(c) <= 2 else e.budget()
     kernels = [('%s<%s, %%d>' % (e.name, S), e.block, e.smem, only) for S in ('false', 'true')]
-    if fp32:
+    short = SHORT.get(tuple(c))
+    if fp32 or short:
         g = GroupEmitter(*c)
         parts.append(g.kernel()[0])
+    if fp32:
         kernels += [('ib_eri_%s<float, %s, %%d>' % (g.tag, S), 'IB_BLOCK', g.smem_bytes, None)
                     for S in ('false', 'true')]
     else:
         kernels *= 2
     parts.append(launcher(e.tag, kernels))
+    if short:
+        parts.append(short_launcher(e.tag, [('ib_eri_%s<double, %s, %d>' % (g.tag, S, MINB_VALUES[short[1]]),
+                                             'IB_BLOCK', g.smem_bytes) for S in ('false', 'true')]))
     return '\n'.join(parts), dict(kind=e.kind, G=e.G, budget=e.budget())
 
 
@@ -485,8 +510,11 @@ def emit_all(outdir, lmax=LMAX_EMIT, ngroups=24):
             regs.append(st)
         parts.append('void ib_register_group_%d(IbClassEntry* table) {' % g)
         for st in regs:
-            parts.append('  table[%d] = IbClassEntry{%d, &ib_launch_%s, &ib_occupancy_%s, %d};'
-                         % (st['cid'], st['cid'], st['tag'], st['tag'], 2 if st['fp32'] else 1))
+            sh = SHORT.get(tuple(int(ch) for ch in st['tag']))
+            parts.append('  table[%d] = IbClassEntry{%d, &ib_launch_%s, &ib_occupancy_%s, %d, %s};'
+                         % (st['cid'], st['cid'], st['tag'], st['tag'], 2 if st['fp32'] else 1,
+                            '&ib_launch_short_%s, &ib_occupancy_short_%s, %d' % (st['tag'], st['tag'], sh[0]) if sh
+                            else 'nullptr, nullptr, -1'))
         parts.append('}')
         _write_if_changed(path, '\n'.join(parts) + '\n')
         written.append(path)

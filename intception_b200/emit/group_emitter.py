@@ -1,5 +1,6 @@
-"""Lane-group ERI kernels of the FP32 tier (and the epilogue that the FP64
-kernels of warp_emitter.py share): G lanes share one contracted quartet.
+"""Lane-group ERI kernels of the FP32 tier and of FP64 quartets with few
+primitives (eri_emitter.SHORT), and the epilogue that the FP64 kernels of
+warp_emitter.py share: G lanes share one contracted quartet.
 
 Each lane of a group owns one Cartesian component s of the "lane side" (the bra
 e-range or the ket f-range, whichever has fewer components) and computes, per
@@ -722,7 +723,7 @@ class GroupEmitter:
         # FP32 tier: growth of an accumulator's error through the HRRs and
         # transforms; a quartet whose error bound already exceeds the
         # tolerance stops its FP32 primitive loop (the final check rejects it)
-        src.append('    const double famp = %s;' % self.amp_expr())
+        src.append('    const double famp = sizeof(R) == 4 ? %s : 0.0;' % self.amp_expr())
         src.append('    (void)famp;')
         src.append('    for (int ab0 = 0; ab0 < kab; ab0 += 64)')
         src.append('    for (int cd0 = 0; cd0 < kcd; cd0 += 64) {')
@@ -746,14 +747,14 @@ class GroupEmitter:
             src.append('        const int ab = ab0 + lst[qa], cd = cd0 + lst[64 + qc];')
             src.append('        if (ab != ab_last) {')
             src.append('          const int ia = (int)(((float)ab + 0.5f) * rkb), ib = ab - ia * kb_;')
-            src.append('          ib_bra_pair(a, g, ia, ib, bp);')
+            src.append('          ib_bra_pair<sizeof(R) == 4>(a, g, ia, ib, bp);')
             src.append('          ab_last = ab;')
             src.append('        }')
             src.append('        const int ic = (int)(((float)cd + 0.5f) * rkd), id = cd - ic * kd_;')
             src.append('        IbPrimQuartet<R> pq;')
             src.append('        double F[%d];' % (L + 1))
             src.append('        if (!ib_prim_quartet<R, %d>(a, g, bp, ic, id, a.boys_tab, F, pq)) continue;' % L)
-            src.append('        {')
+            src.append('        if (sizeof(R) == 4) {')
             src.append('          est += %s;' % self.err_expr())
             src.append('          if (est * famp > a.mixed_tol) break;  // this slice alone already exceeds it')
             src.append('        }')
@@ -779,7 +780,7 @@ class GroupEmitter:
             src.append('            double F[%d];' % (L + 1))
             src.append('            bool live = !(pre && ib_quartet_negligible(lst, qa, qc, a.prim_tol));')
             src.append('            if (live) {')
-            src.append('              ib_bra_pair(a, g, ia, ib, bp);')
+            src.append('              ib_bra_pair<sizeof(R) == 4>(a, g, ia, ib, bp);')
             src.append('              live = ib_prim_quartet<R, %d>(a, g, bp, ic, id, a.boys_tab, F, pq);' % L)
             src.append('            }')
             src.append('            if (live) {')
@@ -787,7 +788,7 @@ class GroupEmitter:
                 src.append('              ps[%d * %d + j] = pq.%s;' % (k, self.G, f))
             for m in range(L + 1):
                 src.append('              ps[%d * %d + j] = (R)F[%d];' % (len(fields) + m, self.G, m))
-            src.append('              est += %s;' % self.err_expr())
+            src.append('              if (sizeof(R) == 4) est += %s;' % self.err_expr())
             src.append('            }')
             src.append('            pz[j] = live ? 1 : 0;  // 0: pair prefactors multiply to zero, or screened out')
             src.append('          }')
@@ -795,7 +796,7 @@ class GroupEmitter:
             src.append('        %s;' % sync)
             # the group's bound so far (its lanes' partial sums): past the
             # tolerance, the rest of this quartet's FP32 work is skipped
-            src.append('        {')
+            src.append('        if (sizeof(R) == 4) {')
             src.append('          double eg = est;')
             if self.packed:
                 src.append('          sb[%d + j] = est;' % self.red_off)
@@ -865,7 +866,7 @@ class GroupEmitter:
         src.append('      ib_sg_sync(SG, sg, sgmask);  // every slice is done with the lists before the next tile')
         src.append('    }')
         # FP32: sum the error bound over the group, reject the quartet if too large
-        src.append('    {')
+        src.append('    if (sizeof(R) == 4) {')
         if self.packed:  # not a power of two: through shared memory
             src.append('      sb[%d + j] = est;' % self.red_off)
             src.append('      __syncwarp(gmask);')
@@ -956,6 +957,16 @@ def launcher(tag, kernels):
     for mi in range(len(MINB_VALUES)):
         for v, (fn, block, smem, only) in enumerate(kernels):
             cases.append((v + 4 * mi, fn % MINB_VALUES[mi if only is None else only], block, smem))
+    return _launcher(tag, cases)
+
+
+def short_launcher(tag, kernels):
+    """The same for the class's short quartets: kernels [(name, threads, shared
+    memory)] for Cartesian and spherical output; variant 0 and 1."""
+    return _launcher('short_' + tag, [(v,) + k for v, k in enumerate(kernels)])
+
+
+def _launcher(tag, cases):
     src = ['static void ib_launch_%s(int variant, int grid, cudaStream_t s, const IbLaunch& a) {' % tag,
            '  switch (variant) {']
     for v, fn, block, smem in cases:

@@ -148,3 +148,35 @@ def test_every_quartet_of_batches_at_the_path_limits(sph, lmax):
         got = eng.compute(out=out).cpu().numpy()
         assert eng.out_size == b.out_off[nq - 1] + np.prod(b.block_dims(nq - 1))
         assert np.abs(got - ref[:eng.out_size]).max() <= tolerance(ref), nq
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('sph', [False, True])
+@pytest.mark.parametrize('lmax', [1, 2, 3])
+def test_short_quartets_of_large_batches(sph, lmax):
+    """Batches of few primitives a shell, large enough that quartets of up to 31
+    primitive quartets (fewer in the wider classes) go to the lane-group
+    kernels: against the same quartets in two batches of half the size, which
+    stay below that size, and against the oracle; screened too, with more and
+    with fewer evaluated quartets than that."""
+    import torch
+    nq = 8192 if lmax == 1 else 32768  # mean K 1.5
+    b = basis.independent_quartet_batch(41, nq, list(range(lmax + 1)), [1, 1, 1, 3], 0.1, 60.0, 5.0, sph)
+    eng = eri.EriEngine(b)
+    got = eng.compute().cpu().numpy()
+    halves = [eri.EriEngine(b.subset(np.arange(i, i + nq // 2))) for i in (0, nq // 2)]
+    want = np.concatenate([e.compute().cpu().numpy() for e in halves])
+    assert np.abs(got - want).max() <= tolerance(want)
+    head = b.subset(np.arange(1500))
+    ref = loader.oracle_batch(head, basis.sph_matrices(6))
+    assert np.abs(got[:head.out_size] - ref).max() <= tolerance(want)
+    two = eri.EriEngine(b.subset(np.concatenate([np.arange(nq)] * 2)))
+    bounds = two.analytic_bounds()
+    for cut in np.quantile(bounds.cpu().numpy(), [0.3, 0.7]):
+        out = torch.full((two.out_size,), 7.0, dtype=torch.float64, device='cuda')
+        two.compute(out=out, bounds=bounds, skip_below=float(cut))
+        d = np.abs(out.cpu().numpy() - np.concatenate([want, want]))
+        off = two.out_off.cpu().numpy()
+        worst = np.maximum.reduceat(d, off)  # packed: largest difference in each quartet's block
+        kept = bounds.cpu().numpy() >= cut
+        assert worst[kept].max() <= tolerance(want) and (worst[~kept] <= 1.000001 * bounds.cpu().numpy()[~kept]).all()
