@@ -61,10 +61,13 @@ constexpr size_t kScratchCap = size_t(4) << 30;  // bytes of generic-kernel scra
 // to kMergedBatch, when the batch has d shells: the sorted pipeline with the
 // class kernels merged into one launch (1 200 quartets 64 / 106 and 97 / 107,
 // 2 400 103 / 110 and 124 / 132; level at 4 096, where the fan-out's register
-// budgets per class start to win).  Without d shells the fan-out is six
-// launches and as fast from 600 quartets on.
+// budgets per class start to win); with few primitives a shell, where a class
+// kernel is over in a few microseconds, up to kMergedShort (K = 1 10 000
+// quartets 146 / 236 us, 25 000 249 / 266; K 1..3 159 / 216, 247 / 247; K 1..6
+// 313 / 249).  Without d shells the fan-out is six launches and as fast from
+// 600 quartets on.
 constexpr int kSmallBatch = 296;
-constexpr int kMergedBatch = 3072;
+constexpr int kMergedBatch = 3072, kMergedShort = 24576;
 // Quartets with few primitive quartets go to the classes' lane-group kernels
 // (IB_SLOT_SHORT) in batches that evaluate at least this many, by the mean
 // contraction length of the basis: below, the warp kernels' latency hides and
@@ -73,8 +76,9 @@ constexpr int kMergedBatch = 3072;
 // 232); K 1..3 50 000 524 / 619, 100 000 l <= 1 323 / 285, l <= 2 879 / 877,
 // 6e5 3.48 / 2.94 ms; K 1..6 100 000 548 / 568, 3e5 915 / 879 (l <= 2 2.13 /
 // 2.17 ms), 1e6 7.54 / 7.41 ms.
+double mean_k(const intception_b200_basis* b) { return b->nshell > 0 ? (double)b->nprim / b->nshell : 1e9; }
 int short_batch(const intception_b200_basis* b) {
-  const double k = b->nshell > 0 ? (double)b->nprim / b->nshell : 1e9;
+  const double k = mean_k(b);
   return k <= 1.6 ? (b->lmax <= 1 ? 1 << 13 : 1 << 15) : k <= 2.25 ? 3 << 15 : 1 << 18;
 }
 constexpr int kRedoGroups = 4;  // redo lists of an l >= 3 batch (dispatch)
@@ -735,13 +739,13 @@ cudaError_t redo_launch(Context* c, cudaStream_t s, const IbLaunch& a, bool sph,
 // Launch the emitted kernels for the given variants and the generic kernel;
 // items/ranges already on the device.  Returns the number of kernels launched.
 int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, int nq, bool fp64_present, bool fp32_present, bool sph,
-             int lmax, bool shorts, int* nlaunch, const ZeroFill* zf = nullptr) {
+             int lmax, int merged_max, bool shorts, int* nlaunch, const ZeroFill* zf = nullptr) {
   // the generic kernel's tickets (zeroed by classify): pair 0 for its range launch, pair 1 + g for redo list g
   int* const tk = c->tickets.as<int>();
   // side streams: one per launch, up to nside (an l <= 2 batch needs 22 of the 40)
   // few l <= 2 quartets: the class kernels as one kernel on the caller's stream
   // (with the HRR check on no quartet is routed to the generic kernel)
-  if (nq <= kMergedBatch && lmax == ib_lmax_emitted && !fp32_present && a.redo && a.hrr_tol > 0.0) {
+  if (nq <= merged_max && lmax == ib_lmax_emitted && !fp32_present && a.redo && a.hrr_tol > 0.0) {
     if (zf) {
       ib_zero_screened<<<std::min(c->nsm * 4, (nq + 255) / 256), 256, 0, s>>>(zf->keys, zf->nq, zf->quartets,
                                                                               zf->shell_l, zf->out_off, sph ? 1 : 0, a.out);
@@ -1366,7 +1370,8 @@ int batch_impl(Context* c, const intception_b200_basis* basis, const int* quarte
   a.hrr_tol = c->hrr_tol;
   if (precision == IB_PREC_MIXED) a.mixed_tol = mixed_tol;
   const ZeroFill zf = {c->keys.as<unsigned>(), nq, quartets, basis->shell_l, out_off};
-  return dispatch(c, s, a, nq, true, precision == IB_PREC_MIXED, spherical != 0, basis->lmax, shorts, nl,
+  return dispatch(c, s, a, nq, true, precision == IB_PREC_MIXED, spherical != 0, basis->lmax,
+                  mean_k(basis) <= 2.25 ? kMergedShort : kMergedBatch, shorts, nl,
                   use_bounds && skip_below > 0.0 ? &zf : nullptr);
 }
 }  // namespace

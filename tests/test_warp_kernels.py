@@ -180,3 +180,19 @@ def test_short_quartets_of_large_batches(sph, lmax):
         worst = np.maximum.reduceat(d, off)  # packed: largest difference in each quartet's block
         kept = bounds.cpu().numpy() >= cut
         assert worst[kept].max() <= tolerance(want) and (worst[~kept] <= 1.000001 * bounds.cpu().numpy()[~kept]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('sph', [False, True])
+def test_merged_kernel_limit_with_few_primitives(sph):
+    """Mean K 1.5: 24576 quartets take the merged kernel, one more a kernel per
+    class; the same values, and the oracle's."""
+    b = basis.independent_quartet_batch(43, 24577, [0, 1, 2], [1, 1, 2, 2], 0.1, 60.0, 5.0, sph)
+    more = eri.EriEngine(b).compute().cpu().numpy()
+    less = eri.EriEngine(b.subset(np.arange(24576))).compute().cpu().numpy()
+    assert np.abs(more[:len(less)] - less).max() <= tolerance(more)
+    head = b.subset(np.arange(1500))
+    ref = loader.oracle_batch(head, basis.sph_matrices(6))
+    assert np.abs(less[:head.out_size] - ref).max() <= tolerance(more)
+    tail = b.subset(np.arange(24300, 24577))
+    assert np.abs(more[-tail.out_size:] - loader.oracle_batch(tail, basis.sph_matrices(6))).max() <= tolerance(more)
