@@ -17,7 +17,9 @@ Paths timed per step, every step a complete pass (screening bounds included):
                  < 1e-18 skipped, the rest in FP64
   mixed          the same screening, FP32 VRR for kept quartets with bound
                  below fp32_below (tuned over a sweep, then measured again),
-                 its rounding-error bound checked, rejected quartets in FP64
+                 its rounding-error bound checked, rejected quartets in FP64;
+                 with no FP32 class kernel in use by default (their FP64
+                 kernels are faster), the FP64 path again
 value = the mixed path (the product's batched path); mixed_over_fp64 compares
 it with fp64_screened, which does the same screening.
 
@@ -489,7 +491,8 @@ def run_c5(args, rank, world, local):
             'metric': 'contracted ERI quartets/s on B200, l<=4 K<=8 screened quartets (sample of the 5e7 batch)',
             'value': nq / (ms_head * 1e-3), 'unit': 'quartets/s', 'n_gpus': world, 'steps': args.steps,
             'warmup': args.warmup, 'ms_per_step': ms_head, 'higher_is_better': True, 'scaling': 'weak',
-            'vs_baseline': None, 'dtype': 'f64+f32' if path == 'precision tiers' else 'f64', 'data': 'synthetic',
+            'vs_baseline': None, 'dtype': 'f64+f32' if path == 'precision tiers' and fp32_tier_on() else 'f64',
+            'data': 'synthetic',
             'config': {'workload': C5_WORKLOAD % batch.nq, 'kept_fraction_of_candidates': frac,
                        'headline_path': path + ' (the fastest path within 1e-10 of exact FP64, measured again)',
                        'prim_tol': PRIM_TOL, 'fp32_below': FP32_BELOW, 'mixed_tol': MIXED_TOL,
@@ -559,7 +562,7 @@ def run_lattice(args, rank, world, local):
     host['mixed'] = out.cpu().numpy()
     rej = eng.fp32_rejected()
     redo_m = eri.last_hrr_redo()
-    nfp32 = int((bounds < FP32_BELOW).sum().item())
+    nfp32 = int((bounds < FP32_BELOW).sum().item()) if fp32_tier_on() else 0
     # the fastest path within 1e-10 of exact FP64, then measured again on its own
     cands = [(ms64, 0.0, 'fp64'), (msp, errp, 'fp64 + primitive screening'), (msm, errm, 'precision tiers')]
     ok = [c for c in cands if c[1] <= ERR_BAR] or cands
@@ -585,7 +588,8 @@ def run_lattice(args, rank, world, local):
             'metric': 'contracted ERI quartets/s on B200, 200-atom l<=3 lattice (screened quartets, sample)',
             'value': nq / (ms * 1e-3), 'unit': 'quartets/s', 'n_gpus': world, 'steps': args.steps,
             'warmup': args.warmup, 'ms_per_step': ms, 'higher_is_better': True, 'scaling': 'weak',
-            'vs_baseline': None, 'dtype': 'f64+f32' if path == 'precision tiers' else 'f64', 'data': 'synthetic',
+            'vs_baseline': None, 'dtype': 'f64+f32' if path == 'precision tiers' and fp32_tier_on() else 'f64',
+            'data': 'synthetic',
             'config': {'workload': LATTICE_WORKLOAD % batch.nq, 'screened_quartets_total': total,
                        'headline_path': path, 'prim_tol': PRIM_TOL, 'fp32_below': FP32_BELOW,
                        'mixed_tol': MIXED_TOL, 'l2': 'outputs %.0f MB per step, larger than L2; no flush'
@@ -737,6 +741,13 @@ def run_twoidx(args, rank, world, local):
                 'roofline': roofline, 'cpu_baseline': cpu, 'e2e': e2e,
                 'gpu_launches': args.steps, 'gpu_launches_per_step': 1, 'clocks': clk.summary()}
         print(json.dumps(line), flush=True)
+
+
+def fp32_tier_on():
+    """Whether any class runs its FP32 kernel by default (the tuned table that
+    the build bakes in); with none, a mixed batch runs in FP64."""
+    with open(os.path.join(ROOT, 'intception_b200', 'tuning.json')) as fh:
+        return any(c.get('fp32', True) for c in json.load(fh)['classes'].values())
 
 
 def profiled_traffic(name):
@@ -937,7 +948,7 @@ def run_eri(args, rank, world, local):
     # ---- FP32-tier setting: a sweep over fp32_below (0 = tier off), then the
     # chosen setting measured on its own as the headline
     sweep = []
-    if not args.no_mixed:
+    if not args.no_mixed and fp32_tier_on():
         for fb in FP32_SWEEP[1:]:
             msx = timed(lambda: screened_step(eri.PREC_MIXED, fb))
             sweep.append({'fp32_below': fb, 'ms_per_step': msx, 'max_abs_err_vs_fp64': err_vs(ref64),

@@ -70,3 +70,25 @@ def test_tuner_times_the_fp32_kernels(monkeypatch):
         for v4 in range(4):
             eri.set_class_minb((2, 1, 1, 1), v4, 0)
     assert len(rel) == 2 * len(autotune.MINB_VALUES) and all(1e-12 < x < 1e-4 for x in rel), rel
+
+
+@pytest.mark.gpu
+def test_bench_names_the_tier_that_runs():
+    """The bench labels a mixed run by the tuned table: with no FP32 class on by
+    default the mixed path gives the FP64 path's bits, with one it does not."""
+    import numpy as np
+    import torch
+    import bench
+    from intception_b200 import basis, eri
+    eng = eri.EriEngine(basis.independent_quartet_batch(3, 4000, [0, 1, 2], [2, 3, 5], 0.1, 40.0, 4.0, True))
+    bounds = torch.ones(eng.nq, dtype=torch.float64, device='cuda')
+    mixed = eng.compute(precision=eri.PREC_MIXED, bounds=bounds, fp32_below=2.0, mixed_tol=1e300).cpu().numpy()
+    assert np.array_equal(mixed, eng.compute().cpu().numpy()) == (not bench.fp32_tier_on())
+
+
+def test_classes_without_an_unrolled_kernel():
+    """Up to g shells only (gg|gg), whose tables exceed a block's shared memory,
+    and (gg|ss), whose accumulators exceed a lane's registers, are left to the
+    generic kernel."""
+    emitted = {c for c, _ in eri_emitter.emitted_classes()}
+    assert set(eri_emitter.canonical_classes(4)) - emitted == {(4, 4, 4, 4), (4, 4, 0, 0)}
