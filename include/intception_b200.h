@@ -146,7 +146,8 @@ typedef struct {
 } intception_b200_basis;
 
 #define IB_PREC_FP64 0  /* every evaluated quartet in FP64 */
-#define IB_PREC_MIXED 1 /* FP32 VRR for quartets whose bound < fp32_below, FP64 otherwise */
+#define IB_PREC_MIXED 1 /* FP32 VRR for quartets whose bound < fp32_below and whose class has its FP32 kernel on
+                           (by default none: see intception_b200_set_class_fp32), FP64 otherwise */
 
 /* Contracted ERIs for nq quartets.  quartets[4*q+0..3] are shell indices
  * (a,b,c,d); quartet q writes its block at out + out_off[q] with a fastest,
@@ -157,10 +158,12 @@ typedef struct {
  * precision is IB_PREC_FP64 and skip_below is 0.  Quartets with
  * bound < skip_below are screened: their block is written as zeros (error <=
  * bound).  With IB_PREC_MIXED, quartets with bound < fp32_below (and at least
- * skip_below) run the VRR in FP32 (Boys, pair setup, contraction sums, HRR and
- * spherical transforms stay FP64) while accumulating a first-order bound on
- * the FP32 rounding error of the finished block; a quartet whose bound exceeds
- * mixed_tol is recomputed in FP64.  Asynchronous on stream (a cudaStream_t;
+ * skip_below) of a class whose FP32 kernel is on run the VRR in FP32 (pair
+ * prefactors, Boys values, square roots and reciprocals' starting values in
+ * float too; contraction sums, HRR and spherical transforms stay FP64) while
+ * accumulating a first-order bound on the FP32 rounding error of the finished
+ * block; a quartet whose bound exceeds mixed_tol is recomputed in FP64.  With
+ * no class on, the default, every quartet is evaluated in FP64.  Asynchronous on stream (a cudaStream_t;
  * NULL = the legacy default stream).  Work buffers are reused between calls:
  * calls on different streams must be ordered by the caller. */
 int intception_b200_eri_batch(const intception_b200_basis *basis, const int *quartets, const long long *out_off,
@@ -274,7 +277,7 @@ int intception_b200_set_class_minb(int cid, int v4, int minb);
  * canonical class cid (cid < 0: every class): 1 where the class has one, 0
  * never (that class's FP32-tier quartets are evaluated in FP64), -1 the
  * default built into the library (the classes whose FP32 kernel the autotuner
- * measured faster).  Waits for the device.  New: no reference counterpart. */
+ * measured faster than the FP64 one: none).  Waits for the device.  New: no reference counterpart. */
 int intception_b200_set_class_fp32(int cid, int on);
 
 /* Waits for the device and returns the device status word of the last batch

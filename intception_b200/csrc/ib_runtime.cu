@@ -57,7 +57,7 @@ constexpr int kKeyBits = 16;
 constexpr size_t kScratchCap = size_t(4) << 30;  // bytes of generic-kernel scratch at most
 // FP64 batches with every l <= 2.  Up to kSmallBatch quartets: the small-batch
 // kernel (us per batch, against the fan-out of one kernel per class: 256
-// quartets of K <= 3 41 / 107, of K <= 6 94 / 108; one block per quartet).  Up
+// quartets of K <= 3 29 / 107, of K <= 6 94 / 108; one block per quartet).  Up
 // to kMergedBatch, when the batch has d shells: the sorted pipeline with the
 // class kernels merged into one launch (1 200 quartets 64 / 106 and 97 / 107,
 // 2 400 103 / 110 and 124 / 132; level at 4 096, where the fan-out's register
@@ -84,10 +84,12 @@ int short_batch(const intception_b200_basis* b) {
 constexpr int kRedoGroups = 4;  // redo lists of an l >= 3 batch (dispatch)
 constexpr int kTickets = 2 * (1 + kRedoGroups);  // generic-kernel ticket pairs: the range launch, each redo list
 // blocks per cluster sharing a heavy generic quartet: a redo list is short and
-// its end waits for its heaviest quartets, so 4; a batch's generic range keeps
-// every block busy, and rank 0's HRRs idle fewer ranks with 2 (l <= 4 sample,
-// 2 000 quartets of one class: (gg|gg) 878 against 1 038 ns per live primitive
-// quartet with 2 and 4, the redo-heavy (gg|ff) 387 against 325)
+// its end waits for its heaviest quartets, so 4; 2 for a batch's generic range,
+// where rank 0's HRRs then idle fewer ranks.  Measured with the inner loop
+// before the Rys form, on batches of one class that keep every block busy:
+// (gg|gg) 878 against 1 038 ns per live primitive quartet with 2 and 4, the
+// redo-heavy (gg|ff) 387 against 325.  A range of a few quartets, as an l <= 4
+// batch's (gg|gg) and (gg|ss) are, was not measured with 4.
 constexpr int kSplitRedo = 4, kSplitRange = 2;
 
 thread_local int tl_status = IB_OK;
@@ -771,7 +773,10 @@ int dispatch(Context* c, cudaStream_t s, const IbLaunch& a, int nq, bool fp64_pr
   // 200-atom lattice sample (1e6 quartets, 65 classes) 5.56 ms with 40, 5.37
   // with 4, 5.77 with one; screened, where few quartets are left, 1.39 / 1.35 /
   // 2.04 ms with 40, 8 and one; the l <= 4 sample (46 quartets a class) 26 / 41
-  // / 84 ms with 40, 4 and one.
+  // / 84 ms with 40, 4 and one.  Above the one-stream limit one stream is the
+  // fastest for every l (ms with 1 / 4 / 64): l <= 2 1.6e6 7.27 / 7.51 / 7.57,
+  // l <= 3 1.6e6 12.27 / 12.42 / 12.55, 4.4e6 31.1 / 32.3 / 32.4, l <= 4 2e6
+  // 49.0 / 51.1 / 50.8, and with 2 % redone at K 1..3 128 with any of them.
   if (nq >= 3 << 19 && !zf)
     nuse = 1;
   else if (nq / nuse >= 8192)

@@ -8,9 +8,10 @@
 // of the class kernel).  A few thousand keep the sort, which brings quartets of
 // one class together (warps of different classes evict one another's code) and
 // the long ones to the front, and run every class in one kernel
-// (ib_merged_kernel).  256 quartets of K <= 3: 107 us with a kernel per class, 31-41
-// here, most of it the dependent loads of one quartet and the launch.  All classes share one register budget there (two blocks
-// per SM), which is why larger batches keep a kernel per class.
+// (ib_merged_kernel).  256 quartets of K <= 3: 107 us with a kernel per class, 29
+// here, most of it the dependent loads of one quartet and the launch.  All classes
+// share one register budget there (two blocks per SM), which is why larger batches
+// keep a kernel per class.
 #pragma once
 #include "ib_eri_device.cuh"
 

@@ -533,10 +533,10 @@ def emit_all(outdir, lmax=LMAX_EMIT, ngroups=24):
     # uses the class's FP32 kernel (where it measured faster than FP64)
     budget = {b[2]['cid']: b[2]['budget'] for b in bodies}
     minb = [[budget.get(cid) or 0] * 2 + [0] * 2 for cid in range(NCLASS_TOTAL)]
-    # at most 8 groups per quartet unless tuned otherwise: measured on the
-    # screened l <= 2 step (3.4 % of 1e6 quartets kept, primitive screening at
-    # 1e-18), a cap of 8 gave 1.18 ms per step against 1.30 uncapped, 1.36 at 2
-    # and 1.64 at 1; a class with many quartets runs one group each anyway
+    # at most 8 groups per quartet unless tuned otherwise (chosen with the
+    # lane-group kernels: screened l <= 2 step 1.18 ms against 1.30 uncapped, 1.36
+    # at 2 and 1.64 at 1; a warp kernel's block has four groups at most); a class
+    # with many quartets runs one group each anyway
     scap = [DEFAULT_SLICE_CAP] * NCLASS_TOTAL
     fp32on = [1] * NCLASS_TOTAL
     tpath = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), 'tuning.json')

