@@ -1099,6 +1099,12 @@ def main():
                                   'screening bounds; the reference C99 is timed in that line\'s cpu_baseline'
                                   % args.workload}))
             return
+        from oracle import loader
+        if (loader.load_ref('sph') if args.workload == 'eri' else loader.load_ref_2idx()) is None:
+            if rank == 0:
+                print(json.dumps({'impl': 'reference', 'unavailable': 'the reference\'s emitted C99 (oracle/_ref) is '
+                                  'built from its source tree, which is not present here'}))
+            return
         if args.workload != 'eri':
             run_twoidx(args, rank, world, 0)
         else:
