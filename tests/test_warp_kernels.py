@@ -1,6 +1,10 @@
 """The warp-per-quartet kernels where their layout changes: batch sizes either
 side of the small-batch and merged-kernel limits, pair counts either side of the
 64-pair tile, and the Rys table's rows and range ends."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -196,3 +200,38 @@ def test_merged_kernel_limit_with_few_primitives(sph):
     assert np.abs(less[:head.out_size] - ref).max() <= tolerance(more)
     tail = b.subset(np.arange(24300, 24577))
     assert np.abs(more[-tail.out_size:] - loader.oracle_batch(tail, basis.sph_matrices(6))).max() <= tolerance(more)
+
+
+CAPTURED = '''
+import sys
+import numpy as np
+import torch
+from intception_b200 import basis, eri
+own = sys.argv[1] == 'own'  # captured on the caller's own stream, not by eri_graph_create
+eng = eri.EriEngine(basis.independent_quartet_batch(8, 500, [0, 1, 2, 3], [4, 6], 0.01, 1e5, 4.0, True))
+out = torch.empty(eng.out_size, dtype=torch.float64, device='cuda')
+ref = eng.compute(out=out).cpu().numpy()
+if own:
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        eng.compute(out=out)
+    replay = g.replay
+else:
+    replay = eng.graph(out).launch
+for nq, l in ((6000, 2), (30000, 5)):
+    eri.EriEngine(basis.independent_quartet_batch(9, nq, [0, 1, l], [1], 0.1, 60.0, 6.0, True)).compute()
+    out.fill_(7.0)
+    replay()
+    assert np.array_equal(out.cpu().numpy(), ref)
+'''
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('how', ['own', 'library'])
+def test_captured_batch_after_larger_batches_in_a_new_process(how):
+    """In a process of its own, where no earlier test has grown the work
+    buffers: a captured batch, by the library or on the caller's stream, replays
+    to the same bits after the library has moved on to larger buffers."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, '-c', CAPTURED, how], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
