@@ -947,7 +947,8 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
   size_t o_it = al(o_c + nprim * sizeof(double));
   size_t o_rg = al(o_it + nblk * sizeof(IbItem));
   size_t o_T[4];
-  size_t cur = al(o_rg + kNRanges * sizeof(int));
+  constexpr int nranges = IB_SLOT_LONG_END;  // the class and generic ranges
+  size_t cur = al(o_rg + nranges * sizeof(int));
   for (int i = 0; i < 4; ++i) {
     o_T[i] = cur;
     cur = al(cur + tsize[i] * sizeof(double));
@@ -1047,7 +1048,7 @@ int dropin(DropShell* sh, bool sph, double* output_array) {
           it.off = (long long)b * cart_block;
           hit[b] = it;
         }
-  std::memset(hrg, 0, kNRanges * sizeof(int));
+  std::memset(hrg, 0, nranges * sizeof(int));
   const bool emitted = c->table[cidx].launch != nullptr && !route;
   if (emitted) {
     hrg[2 * cidx] = 0;
